@@ -133,12 +133,7 @@ int jf_int8_add_meanvar_noalloc(const void* x1, int x1_dtype, const int8_t* q2, 
  * and differ in operand layout and epilogue.  Scale tensors are addressed with explicit element strides so both the
  * natural [rows/32, cols/32] layout and the transposed copies the reference passes are accepted without a copy.
  *
- * op16 / op16_bytes (all three): optional scratch for exact fp16 copies of both operands, 2 * (M*K + N*K) bytes, 16-byte
- * aligned.  When it is given (and large enough) the GEMM first writes the two copies ([M,K] and [N,K], transposing where the
- * operand is stored [K, rows]) and then runs on them with tcgen05.mma kind::f16, whose fp32 accumulator already holds
- * float(I_p): the consumers skip the int32 -> fp32 conversion that bounds the int8-operand kernel.  Results are bit-identical
- * either way (every partial sum is an integer below 2^24).  It pays for large GEMMs only (8192^3: 1.75 -> 1.49 ms including the
- * conversion passes); jf_igemm_op16_bytes says when.  NULL / 0 selects the int8-operand kernel.
+ * op16 / op16_bytes (all three): accepted and not used (the operands are always read in place).
  * ---------------------------------------------------------------------------------------------------------- */
 
 /* Output selector of the re-quantising GEMMs. */
@@ -186,8 +181,7 @@ int jf_igemm_wgrad(const int8_t* g, int g_transposed, const int8_t* x, const voi
  * size `scratch`.  Host-only; launches nothing. */
 int jf_igemm_wgrad_plan(int64_t M, int64_t N, int64_t K, int split_k);
 
-/* Size of the fp16 operand scratch (bytes) for a GEMM of these dimensions if the fp16-operand path is expected to pay for its
- * conversion passes, else 0.  Host-only; launches nothing.  No counterpart in the reference. */
+/* Bytes of operand scratch worth passing as `op16` to a GEMM of these dimensions: always 0. */
 int64_t jf_igemm_op16_bytes(int64_t M, int64_t N, int64_t K);
 
 /* Plain int8 x int8 -> int32 product C[M,N] = A[M,K] * B[N,K]^T (test/diagnostic entry point).

@@ -6,16 +6,11 @@
 // followed by a per-32x32-block re-quantisation (or a dense fp16/fp32 store) of acc.
 //
 // Mapping to the hardware
-//   * CTA tile 128 x 128, one CTA per SM, persistent over a static list of (tile, K-split) work items.
-//   * 19 warps: 16 consumers, 1 TMA producer (one lane), 2 MMA issuers (one lane each).
-//   * producer: a 128-byte-swizzled 128 x 128 B box per operand per stage = four K blocks; a 4-stage mbarrier ring (128 KB).
-//   * issuers: tcgen05.mma kind::i8 has K = 32 = one quantisation block, so every K block is ONE 128x128x32 MMA with
-//     accumulation disabled.  Tensor memory (512 columns) holds two groups of two 128-column accumulators; the four K blocks
-//     of a stage form two pairs, pair g goes to group g and is issued by issuer g with one tcgen05.commit.
-//   * consumers: warp w reads TMEM lanes 32*(w%4).. (rows) and columns 32*(w/4).. of every accumulator with tcgen05.ld (a
-//     thread = one row of one quantisation block), converts int32 -> fp32 and does the scale FMA into 32 fp32 registers.  This
-//     CUDA-core work, not the tensor core, bounds the kernel.  Scale products are fetched one per lane for 8 K blocks at a
-//     time and broadcast by shuffle.
+//   * CTA tile 128 x 64, two CTAs per SM, persistent over a static list of (tile, K-split) work items.
+//   * producer: one 128-byte-swizzled box per operand per stage = four K blocks; a 4-stage mbarrier ring (96 KB).
+//   * issuer: tcgen05.mma kind::i8 has K = 32 = one quantisation block, so every K block is ONE 128x64x32 MMA with accumulation disabled.
+//   * consumers: tcgen05.ld (a thread = one row of one quantisation block), int32 -> fp32, scale FMA into 32 fp32 registers.  This
+//     CUDA-core work, not the tensor core, bounds the kernel.
 //   * operands are consumed in place in either orientation: K-major (row-major [rows, K]) or MN-major (row-major
 //     [K, rows]) through the UMMA descriptor major bits, so no transposed copy of W, dY or X is ever materialised.
 //   * epilogue: a 32x32 block = 32 lanes x 32 thread-local values; absmax is a local max + one redux.sync.
@@ -31,15 +26,16 @@
 
 namespace jf {
 
-constexpr int BM = 128, BN = 128;
+constexpr int BM = 128, BN = 64;                // CTA tile; two CTAs share an SM
 constexpr int KB_PER_STAGE = 4;                 // 32-wide K blocks per pipeline stage (128 bytes of K)
 constexpr int STAGES = 4;
-constexpr int STAGE_BYTES = 128 * 128;          // one operand tile
-constexpr int TMEM_COLS = 512;
-constexpr size_t GEMM_SMEM = 2 * STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
-constexpr size_t GEMM_SMEM_F16OPS = 2 * 3 * 2 * STAGE_BYTES + 1024 + 256;   // three stages of two boxes per operand
+constexpr int A_BYTES = BM * 128, B_BYTES = BN * 128, STAGE_BYTES = A_BYTES + B_BYTES;
+constexpr int CONSUMER_WARPS = 8;
+constexpr int GEMM_THREADS = (CONSUMER_WARPS + 2) * 32;
+constexpr int TMEM_COLS = 4 * BN;               // four accumulators
+constexpr size_t GEMM_SMEM = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 128 /*barriers*/;
 constexpr long long DRAIN_BUDGET_CLOCKS = 20000000LL;   // ~10 ms: abort-path wait for copies / MMAs already in flight
-constexpr long long WAIT_BUDGET_CLOCKS = 4000000000LL;  // ~2 s at 2 GHz
+constexpr uint32_t WAIT_BUDGET_CLOCKS = 4000000000u;    // ~2 s at 2 GHz (32-bit clock)
 
 enum GemmMode : int {
     MODE_INT8 = 0,      // int8 payload + fp16 scales
@@ -64,26 +60,6 @@ struct GemmParams {
 
 __device__ int g_gemm_error = 0;   // 0 = ok; otherwise the code of the first wait that expired
 
-// Wait for a barrier phase, giving up after WAIT_BUDGET_CLOCKS.  SUSPEND = true (producer and issuer warps): every try lets the
-// hardware park the thread for up to 2 us; SUSPEND = false (consumers): plain try_wait polling.  (An additional __nanosleep of
-// 40-250 ns between the tries of the producer / issuer warps measured 2-4 % slower.)
-template <bool SUSPEND = false>
-__device__ __forceinline__ bool bounded_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
-    if (ptx::mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    for (uint32_t it = 0;; ++it) {
-        if (SUSPEND ? ptx::mbar_try_wait_hint(bar, parity, 2000u) : ptx::mbar_try_wait(bar, parity)) return true;
-        if ((it & (SUSPEND ? 31u : 255u)) == (SUSPEND ? 31u : 255u)) {
-            if (*abort_flag) return false;
-            if (clock64() - t0 > WAIT_BUDGET_CLOCKS) {
-                *abort_flag = code;
-                atomicCAS(&g_gemm_error, 0, code);
-                return false;
-            }
-        }
-    }
-}
-
 // Abort path: wait for a barrier phase that operations already in flight will complete, without touching the abort state.
 __device__ __forceinline__ void drain_wait(uint64_t* bar, uint32_t parity) {
     const long long t0 = clock64();
@@ -93,23 +69,11 @@ __device__ __forceinline__ void drain_wait(uint64_t* bar, uint32_t parity) {
 
 // ---------------------------------------------------------------------------------------------------------
 // Consumer arithmetic.  acc is kept as packed pairs of fp32 so the scale FMA can use the two-wide fma.rn.f32x2.
-// int32 -> fp32 (cvt.rn.f32.s32) is exact: |I| <= 32*127^2 < 2^22.  (Building the float with an integer add of 0x4B400000 and
-// a subtraction of 1.5*2^23 instead, for all or for every other pair, measured slower: the add runs on the same pipe.)
+// int32 -> fp32 (cvt.rn.f32.s32) is exact: |I| <= 32*127^2 < 2^22.  (Building the float with an integer multiply-add of 0x4B400000 on the
+// FMA pipe and a subtraction of 1.5*2^23 for 1/8, 1/4 or 1/2 of the values, to relieve the ALU pipe, measured 1-15 % slower.)
 // CONV_INT32 adds the raw integers instead: the plain int32 GEMM behind jf_igemm_int32.
 // ---------------------------------------------------------------------------------------------------------
-enum ConvMode : int { CONV_I2F = 0, CONV_INT32 = 1, CONV_F16OPS = 2 };
-
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
+enum ConvMode : int { CONV_I2F = 0, CONV_INT32 = 1 };
 
 // acc2[j] (16 packed pairs) += s * float(r[2j], r[2j+1]) for the 32 int32 values in r
 template <int CONV>
@@ -122,103 +86,127 @@ __device__ __forceinline__ void scale_accumulate(uint64_t (&acc2)[16], const uin
         }
         return;
     }
-    const uint64_t s2 = pack2(s, s);
-    if constexpr (CONV == CONV_F16OPS) {      // the accumulator already holds float(I_p)
+    const uint64_t s2 = f2_pack(s, s);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) acc2[j] = fma2(s2, pack2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1])), acc2[j]);
-    } else {
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-            acc2[j] = fma2(s2, pack2(__int2float_rn((int)r[2 * j]), __int2float_rn((int)r[2 * j + 1])), acc2[j]);
+    for (int j = 0; j < 16; ++j) {
+        const uint64_t v = f2_pack(__int2float_rn((int)r[2 * j]), __int2float_rn((int)r[2 * j + 1]));
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc2[j]) : "l"(s2), "l"(v));
     }
 }
 
-// Re-quantise / convert one 32x32 block held as 32 lanes x 32 values and store it.
-__device__ __forceinline__ void store_block(const GemmParams& p, const float (&ab)[32], int64_t row, int64_t col, int64_t rowblk,
+// Re-quantise / convert one 32x32 block held as 32 lanes x 16 packed pairs and store it.  Two values per instruction throughout.
+__device__ __forceinline__ void store_block(const GemmParams& p, const uint64_t (&acc2)[16], int64_t row, int64_t col, int64_t rowblk,
                                             int64_t colblk, int64_t split, int lane) {
     if (p.mode == MODE_INT32) {
         int4* dst = reinterpret_cast<int4*>(p.out_i32 + row * p.N + col);
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
-            dst[k] = make_int4(__float_as_int(ab[4 * k]), __float_as_int(ab[4 * k + 1]), __float_as_int(ab[4 * k + 2]), __float_as_int(ab[4 * k + 3]));
+        for (int k = 0; k < 8; ++k) dst[k] = make_int4((int)acc2[2 * k], (int)(acc2[2 * k] >> 32), (int)acc2[2 * k + 1], (int)(acc2[2 * k + 1] >> 32));
     } else if (p.mode == MODE_F32) {
         float4* dst = reinterpret_cast<float4*>(p.out32 + (split * p.M + row) * p.N + col);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) dst[k] = make_float4(ab[4 * k], ab[4 * k + 1], ab[4 * k + 2], ab[4 * k + 3]);
+        for (int k = 0; k < 8; ++k) {
+            float4 v;
+            f2_unpack(acc2[2 * k], v.x, v.y);
+            f2_unpack(acc2[2 * k + 1], v.z, v.w);
+            dst[k] = v;
+        }
     } else if (p.mode == MODE_F16) {
         int4* dst = reinterpret_cast<int4*>(p.out16 + row * p.N + col);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             __half2 h[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) h[u] = __floats2half2_rn(ab[8 * k + 2 * u], ab[8 * k + 2 * u + 1]);
+            for (int u = 0; u < 4; ++u) {
+                float lo, hi;
+                f2_unpack(acc2[4 * k + u], lo, hi);
+                h[u] = __floats2half2_rn(lo, hi);
+            }
             dst[k] = *reinterpret_cast<int4*>(h);
         }
     } else {
         float m = 0.f;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) m = fmaxf(m, fabsf(ab[j]));
+        for (int j = 0; j < 16; ++j) {
+            float lo, hi;
+            f2_unpack(acc2[j], lo, hi);
+            m = fmaxf(m, fmaxf(fabsf(lo), fabsf(hi)));
+        }
         const float amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
         const __half sc16 = __float2half_rn(__fdiv_rn(amax, 127.0f));
         const Divisor d = make_divisor(amax);
         const bool zero = (amax == 0.f);
-        uint32_t words[8];
-        // One decision per warp each: the exact-quotient fast path is valid for the whole block (same divisor in every lane),
-        // and only stochastic rounding can leave [-127, 127] (127 + noise -> 128), so only it needs the clamp.
+        const uint64_t c127 = f2_pack(127.0f, 127.0f), inv2 = f2_pack(d.inv, d.inv), negb2 = f2_pack(-d.b, -d.b);
+        const uint64_t magic2 = f2_pack(12582912.0f, 12582912.0f), nmagic2 = f2_pack(-12582912.0f, -12582912.0f);
+        const float scf = __half2float(sc16);
+        const uint64_t scf2 = f2_pack(scf, scf);
+        // One decision per warp each: the exact-quotient fast path is valid for the whole block (same divisor in every lane), and
+        // only stochastic rounding can leave [-127, 127], so only it needs the clamp.
         const bool fast = __all_sync(0xffffffffu, d.fast || zero);
-        auto quantise_all = [&](auto fast_c, auto sr_c) {
-            constexpr bool FAST = decltype(fast_c)::value, SRND = decltype(sr_c)::value;
+        auto quantise_all = [&](auto fast_c, auto sr_c, auto deq_c) {
+            constexpr bool FAST = decltype(fast_c)::value, SRND = decltype(sr_c)::value, DEQ = decltype(deq_c)::value;
+            uint32_t words[8];
 #pragma unroll
             for (int k8 = 0; k8 < 4; ++k8) {      // 8 elements = one Philox call
-                float nz[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                uint64_t nz2[4] = {0ull, 0ull, 0ull, 0ull};
                 if (SRND) {
                     if (p.noise) {
                         const float4 n0 = __ldg(reinterpret_cast<const float4*>(p.noise + row * p.N + col + 8 * k8));
                         const float4 n1 = __ldg(reinterpret_cast<const float4*>(p.noise + row * p.N + col + 8 * k8 + 4));
-                        nz[0] = n0.x; nz[1] = n0.y; nz[2] = n0.z; nz[3] = n0.w; nz[4] = n1.x; nz[5] = n1.y; nz[6] = n1.z; nz[7] = n1.w;
+                        nz2[0] = f2_pack(n0.x, n0.y); nz2[1] = f2_pack(n0.z, n0.w); nz2[2] = f2_pack(n1.x, n1.y); nz2[3] = f2_pack(n1.z, n1.w);
                     } else {
-                        philox_noise8((uint64_t)(row * p.N + col + 8 * k8), p.keys, p.offset, nz);
+                        philox_noise8x2((uint64_t)(row * p.N + col + 8 * k8), p.keys, p.offset, nz2);
                     }
                 }
+                uint32_t bits[8], h16[4];
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    uint32_t bts[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const float a127 = __fmul_rn(127.0f, ab[8 * k8 + 4 * h + u]);
-                        float v;
-                        if (FAST) {
-                            const float q0 = __fmul_rn(a127, d.inv);
-                            v = __fmaf_rn(__fmaf_rn(-d.b, q0, a127), d.inv, q0);
-                        } else {
-                            v = __fdiv_rn(a127, d.b);
-                        }
-                        if (SRND) v = fminf(fmaxf(__fadd_rn(v, nz[4 * h + u]), -127.f), 127.f);
-                        bts[u] = __float_as_uint(__fadd_rn(v, 12582912.0f));     // round to nearest even; the low byte is the payload
+                for (int u = 0; u < 4; ++u) {
+                    const uint64_t a127 = f2_mul(c127, acc2[4 * k8 + u]);
+                    uint64_t v2;
+                    if (FAST) {
+                        v2 = f2_div_fast(a127, inv2, negb2);
+                    } else {
+                        float lo, hi;
+                        f2_unpack(a127, lo, hi);
+                        v2 = f2_pack(__fdiv_rn(lo, d.b), __fdiv_rn(hi, d.b));
                     }
-                    words[2 * k8 + h] = zero ? 0u : __byte_perm(__byte_perm(bts[0], bts[1], 0x0040), __byte_perm(bts[2], bts[3], 0x0040), 0x5410);
+                    if (SRND) {
+                        float lo, hi;
+                        f2_unpack(f2_add(v2, nz2[u]), lo, hi);
+                        v2 = f2_pack(fminf(fmaxf(lo, -127.f), 127.f), fminf(fmaxf(hi, -127.f), 127.f));
+                    }
+                    v2 = f2_add(v2, magic2);                   // round to nearest even; the low byte is the payload
+                    float lo, hi;
+                    if (DEQ) {
+                        f2_unpack(f2_mul(f2_add(v2, nmagic2), scf2), lo, hi);      // payload x scale, exact in fp32
+                        const __half2 h = __floats2half2_rn(lo, hi);
+                        h16[u] = zero ? 0u : *reinterpret_cast<const uint32_t*>(&h);
+                    } else {
+                        f2_unpack(v2, lo, hi);
+                        bits[2 * u] = __float_as_uint(lo); bits[2 * u + 1] = __float_as_uint(hi);
+                    }
                 }
+                if (DEQ) {
+                    reinterpret_cast<uint4*>(p.out16 + row * p.N + col)[k8] = make_uint4(h16[0], h16[1], h16[2], h16[3]);
+                } else {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        words[2 * k8 + h] = zero ? 0u : __byte_perm(__byte_perm(bits[4 * h], bits[4 * h + 1], 0x0040),
+                                                                    __byte_perm(bits[4 * h + 2], bits[4 * h + 3], 0x0040), 0x5410);
+                }
+            }
+            if (!DEQ) {
+                int4* dst = reinterpret_cast<int4*>(p.out8 + row * p.N + col);
+                dst[0] = make_int4(words[0], words[1], words[2], words[3]);
+                dst[1] = make_int4(words[4], words[5], words[6], words[7]);
+                if (lane == 0) p.out_scale[rowblk * (p.N / QB) + colblk] = sc16;
             }
         };
         using T_ = std::true_type; using F_ = std::false_type;
-        if (fast) { if (p.stochastic) quantise_all(T_{}, T_{}); else quantise_all(T_{}, F_{}); }
-        else      { if (p.stochastic) quantise_all(F_{}, T_{}); else quantise_all(F_{}, F_{}); }
-        if (p.mode == MODE_INT8) {
-            int4* dst = reinterpret_cast<int4*>(p.out8 + row * p.N + col);
-            dst[0] = make_int4(words[0], words[1], words[2], words[3]);
-            dst[1] = make_int4(words[4], words[5], words[6], words[7]);
-            if (lane == 0) p.out_scale[rowblk * (p.N / QB) + colblk] = sc16;
-        } else {   // MODE_DEQ16
-            const float scf = __half2float(sc16);
-            int4* dst = reinterpret_cast<int4*>(p.out16 + row * p.N + col);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                __half h[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) h[u] = deq16(sbyte(words[2 * k + (u >> 2)], u & 3), scf);
-                dst[k] = *reinterpret_cast<int4*>(h);
-            }
-        }
+        auto rounding = [&](auto fast_c) {
+            if (p.mode == MODE_INT8) { if (p.stochastic) quantise_all(fast_c, T_{}, F_{}); else quantise_all(fast_c, F_{}, F_{}); }
+            else                     { if (p.stochastic) quantise_all(fast_c, T_{}, T_{}); else quantise_all(fast_c, F_{}, T_{}); }
+        };
+        if (fast) rounding(T_{}); else rounding(F_{});
     }
 }
 
@@ -262,128 +250,22 @@ static EncodeTiledFn get_encode_fn() {
     return fn;
 }
 
-// 2-D uint8 tensor [outer, inner] with row pitch `pitch` bytes; box 128 x 128, 128-byte swizzle, zero fill outside.
-static int make_map(CUtensorMap* map, const void* base, int64_t inner, int64_t outer, int64_t pitch) {
+// 2-D uint8 tensor [outer, inner], box box_inner x box_outer, swizzle of the box's width (64 or 128 bytes), zero fill outside.
+static int make_map(CUtensorMap* map, const void* base, int64_t inner, int64_t outer, int box_inner, int box_outer) {
     EncodeTiledFn fn = get_encode_fn();
     if (!fn) return JF_ERR_UNSUPPORTED;
     const cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer};
-    const cuuint64_t strides[1] = {(cuuint64_t)pitch};
-    const cuuint32_t box[2] = {128, 128};
+    const cuuint64_t strides[1] = {(cuuint64_t)inner};
+    const cuuint32_t box[2] = {(cuuint32_t)box_inner, (cuuint32_t)box_outer};
     const cuuint32_t estr[2] = {1, 1};
     CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, box_inner == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         g_last_cuda_error = (int)r;
         return JF_ERR_LAUNCH;
     }
     return JF_OK;
-}
-
-// 2-D fp16 tensor [outer, inner]: box 64 elements (128 B) x 128 rows, 128-byte swizzle, zero fill outside.
-static int make_map_f16(CUtensorMap* map, const void* base, int64_t inner, int64_t outer) {
-    EncodeTiledFn fn = get_encode_fn();
-    if (!fn) return JF_ERR_UNSUPPORTED;
-    const cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer};
-    const cuuint64_t strides[1] = {(cuuint64_t)(inner * 2)};
-    const cuuint32_t box[2] = {64, 128};
-    const cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        g_last_cuda_error = (int)r;
-        return JF_ERR_LAUNCH;
-    }
-    return JF_OK;
-}
-
-// exact fp16 copy of an int8 tensor (16 elements per thread)
-__global__ void int8_to_f16_kernel(const int8_t* __restrict__ q, int64_t count16, __half* __restrict__ out) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count16) return;
-    const int4 v = __ldg(reinterpret_cast<const int4*>(q) + i);
-    const uint32_t w[4] = {(uint32_t)v.x ^ 0x80808080u, (uint32_t)v.y ^ 0x80808080u, (uint32_t)v.z ^ 0x80808080u, (uint32_t)v.w ^ 0x80808080u};
-    const __half2 bias = __floats2half2_rn(1152.f, 1152.f);
-    uint32_t o[8];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const uint32_t lo = __byte_perm(w[k], 0x64646464u, 0x5140), hi = __byte_perm(w[k], 0x64646464u, 0x5342);
-        const __half2 a = __hsub2_rn(*reinterpret_cast<const __half2*>(&lo), bias), b = __hsub2_rn(*reinterpret_cast<const __half2*>(&hi), bias);
-        o[2 * k] = *reinterpret_cast<const uint32_t*>(&a); o[2 * k + 1] = *reinterpret_cast<const uint32_t*>(&b);
-    }
-    uint4* dst = reinterpret_cast<uint4*>(out) + 2 * i;
-    dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-    dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
-}
-
-// exact fp16 copy of the TRANSPOSE of an int8 tensor: q [R, C] row-major -> out [C, R] row-major.  A CTA moves a 128 x 128 tile
-// through shared memory (16-byte chunks XOR-permuted per 16-row group, so that the column reads are bank-conflict free); a thread
-// gathers a 16-row x 4-column patch, transposes it with byte permutes and writes 16 fp16 (32 bytes) of each of 4 output rows:
-// 8 neighbouring threads complete 256 contiguous bytes.
-__global__ void __launch_bounds__(256) int8_to_f16_transposed_kernel(const int8_t* __restrict__ q, int64_t R, int64_t C, __half* __restrict__ out) {
-    __shared__ __align__(16) uint32_t tile[128 * 128 / 4];
-    const int64_t R0 = (int64_t)blockIdx.y * 128, C0 = (int64_t)blockIdx.x * 128;
-    const int t = threadIdx.x;
-    {
-        const int chunk = t & 7;
-#pragma unroll
-        for (int pass = 0; pass < 4; ++pass) {
-            const int row = (t >> 3) + 32 * pass;
-            int4 v = make_int4(0, 0, 0, 0);
-            if (R0 + row < R && C0 + 16 * chunk < C) v = __ldg(reinterpret_cast<const int4*>(q + (R0 + row) * C + C0 + 16 * chunk));
-            *reinterpret_cast<int4*>(tile + row * 32 + 4 * (chunk ^ ((row >> 4) & 7))) = v;
-        }
-    }
-    __syncthreads();
-    const int warp = t >> 5, lane = t & 31;
-    const int i = lane & 7, cg = 4 * warp + (lane >> 3);
-    if (R0 + 16 * i >= R || C0 + 4 * cg >= C) return;
-    const __half2 bias = __floats2half2_rn(1152.f, 1152.f);
-    uint32_t colw[4][4];
-#pragma unroll
-    for (int g = 0; g < 4; ++g) {
-        uint32_t w[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) w[k] = tile[(16 * i + 4 * g + k) * 32 + 4 * ((cg >> 2) ^ i) + (cg & 3)];
-        // 4x4 byte transpose: colw[j][g] = rows 4g..4g+3 of column j
-        const uint32_t t0 = __byte_perm(w[0], w[1], 0x5140), t1 = __byte_perm(w[2], w[3], 0x5140);
-        const uint32_t t2 = __byte_perm(w[0], w[1], 0x7362), t3 = __byte_perm(w[2], w[3], 0x7362);
-        colw[0][g] = __byte_perm(t0, t1, 0x5410); colw[1][g] = __byte_perm(t0, t1, 0x7632);
-        colw[2][g] = __byte_perm(t2, t3, 0x5410); colw[3][g] = __byte_perm(t2, t3, 0x7632);
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        uint32_t o[8];
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-            const uint32_t wx = colw[j][g] ^ 0x80808080u;
-            const uint32_t lo = __byte_perm(wx, 0x64646464u, 0x5140), hi = __byte_perm(wx, 0x64646464u, 0x5342);
-            const __half2 a = __hsub2_rn(*reinterpret_cast<const __half2*>(&lo), bias), b = __hsub2_rn(*reinterpret_cast<const __half2*>(&hi), bias);
-            o[2 * g] = *reinterpret_cast<const uint32_t*>(&a); o[2 * g + 1] = *reinterpret_cast<const uint32_t*>(&b);
-        }
-        uint4* dst = reinterpret_cast<uint4*>(out + (C0 + 4 * cg + j) * R + R0 + 16 * i);
-        dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-        dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
-    }
-}
-
-// Fill the fp16 operand copies of one GEMM: a16 [M,K] from a ([M,K], or [K,M] when a_transposed), b16 [N,K] likewise.
-static int fill_f16_operands(const int8_t* a, bool a_transposed, const int8_t* b, bool b_transposed, int64_t M, int64_t N, int64_t K,
-                             __half* a16, __half* b16, cudaStream_t st) {
-    auto one = [&](const int8_t* src, bool transposed, int64_t rows, __half* dst) {     // dst [rows, K]
-        if (transposed) {   // src is [K, rows]
-            const dim3 grid((unsigned)((rows + 127) / 128), (unsigned)((K + 127) / 128));
-            int8_to_f16_transposed_kernel<<<grid, 256, 0, st>>>(src, K, rows, dst);
-        } else {
-            const int64_t n16 = rows * K / 16;
-            int8_to_f16_kernel<<<(unsigned)((n16 + 255) / 256), 256, 0, st>>>(src, n16, dst);
-        }
-    };
-    if ((K + 127) / 128 > 65535) return JF_ERR_SHAPE;
-    one(a, a_transposed, M, a16);
-    one(b, b_transposed, N, b16);
-    return check_launch();
 }
 
 struct DeviceInfo {
@@ -409,15 +291,23 @@ static int device_info(DeviceInfo** out) {
 
 #include "gemm_launch.inc"
 
+// Number of K ranges of a weight-gradient GEMM.  An SM works through ceil(items / SMs) items, two at a time (one alone reaches ~0.7 of
+// their common rate); an item costs its K blocks (~0.11 us each) plus ~7 K blocks' worth of start and epilogue; a split adds a kernel and
+// the fp32 partials' way through memory (~4 TB/s: they are mostly served by L2).  Ranges keep at least 16 K blocks.
+// [768 x 2304], K = 12288: 216 tiles leave a quarter of the 296 CTA slots idle; two ranges take 76 instead of 92 us.
 static int plan_splits(int64_t M, int64_t N, int64_t K, int split_k, int sm_count, int64_t* per_out) {
     const int64_t nkb = K / QB;
     int64_t s = split_k;
     if (s <= 0) {
         const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-        s = sm_count / tiles;
-        const int64_t cap = nkb / 16;   // keep at least 16 K blocks per range
-        if (s > cap) s = cap;
-        if (s < 1) s = 1;
+        double best = 0.0;
+        s = 1;
+        for (int64_t c = 1; c <= 8 && (c == 1 || nkb / c >= 16); ++c) {
+            const int64_t per = (nkb + c - 1) / c, rounds = (tiles * c + sm_count - 1) / sm_count;
+            double cost = (double)rounds * (double)(per + 7) * (rounds == 1 ? 1.4 : 1.0);
+            if (c > 1) cost += (3.0 + (double)c * (double)M * (double)N * 8.0 / 4e6) / 0.11;
+            if (c == 1 || cost < best) { best = cost; s = c; }
+        }
     }
     if (s > nkb) s = nkb;
     const int64_t per = (nkb + s - 1) / s;
@@ -428,11 +318,6 @@ static int plan_splits(int64_t M, int64_t N, int64_t K, int split_k, int sm_coun
 }  // namespace jf
 
 using namespace jf;
-
-// the fp16-operand path is taken when the caller handed in enough scratch for both operand copies
-static inline bool use_op16(const void* op16, int64_t op16_bytes, int64_t M, int64_t N, int64_t K) {
-    return op16 != nullptr && aligned16(op16) && op16_bytes >= 2 * (M * K + N * K);
-}
 
 static inline int check_gemm_dims(int64_t M, int64_t N, int64_t K) {
     if (!mult32(M) || !mult32(N) || !mult32(K)) return JF_ERR_SHAPE;
@@ -463,24 +348,13 @@ int jf_igemm_forward(const int8_t* x, const int8_t* w, const void* sx, int64_t s
     } else {
         return JF_ERR_ARG;
     }
-    if (use_op16(op16, op16_bytes, M, N, K)) {
-        __half* a16 = (__half*)op16;
-        __half* b16 = a16 + M * K;
-        if (int e = fill_f16_operands(x, false, w, false, M, N, K, a16, b16, (cudaStream_t)stream)) return e;
-        return launch_f16ops(a16, b16, p, (cudaStream_t)stream);
-    }
+    (void)op16; (void)op16_bytes;
     return launch_fwd(x, w, p, (cudaStream_t)stream);
 }
 
-/* Bytes of fp16 operand scratch a GEMM with these dimensions needs for the fp16-operand path (2 * (M*K + N*K)), or 0 when that
- * path is not expected to pay for its conversion passes.  Model: the kernel saves ~20 % of a GEMM that runs at ~630e12 ops/s; the
- * passes move 3 bytes per operand element at ~5e12 B/s plus two launches. */
-int64_t jf_igemm_op16_bytes(int64_t M, int64_t N, int64_t K) {
-    if (check_gemm_dims(M, N, K)) return 0;
-    const double gain = 0.2 * 2.0 * (double)M * (double)N * (double)K / 630e12;
-    const double cost = 3.0 * ((double)M * K + (double)N * K) / 5e12 + 4e-6;
-    return gain > 1.5 * cost ? 2 * (M * K + N * K) : 0;
-}
+/* Bytes of operand scratch worth passing to a GEMM with these dimensions: none, the kernel reads the int8 operands in place
+ * (the `op16` arguments of the GEMM entry points are accepted and not used). */
+int64_t jf_igemm_op16_bytes(int64_t, int64_t, int64_t) { return 0; }
 
 int jf_igemm_dgrad(const int8_t* g, const int8_t* w, const void* sg, int64_t sg_stride_m, int64_t sg_stride_k, const void* sw,
                    int64_t sw_stride_k, int64_t sw_stride_n, int64_t M, int64_t N, int64_t K, int out_mode, int8_t* dx8, void* sdx,
@@ -505,12 +379,7 @@ int jf_igemm_dgrad(const int8_t* g, const int8_t* w, const void* sg, int64_t sg_
     } else {
         return JF_ERR_ARG;
     }
-    if (use_op16(op16, op16_bytes, M, N, K)) {
-        __half* a16 = (__half*)op16;
-        __half* b16 = a16 + M * K;
-        if (int e = fill_f16_operands(g, false, w, true, M, N, K, a16, b16, (cudaStream_t)stream)) return e;
-        return launch_f16ops(a16, b16, p, (cudaStream_t)stream);
-    }
+    (void)op16; (void)op16_bytes;
     return launch_dgrad_layout(g, w, p, (cudaStream_t)stream);
 }
 
@@ -538,12 +407,8 @@ int jf_igemm_wgrad(const int8_t* g, int g_transposed, const int8_t* x, const voi
     p.sa = (const __half*)sg; p.sa_sm = sg_stride_m; p.sa_sk = sg_stride_k;
     p.sb = (const __half*)sx; p.sb_sn = sx_stride_n; p.sb_sk = sx_stride_k;
     cudaStream_t st = (cudaStream_t)stream;
-    const bool f16 = use_op16(op16, op16_bytes, M, N, K);
-    __half* a16 = (__half*)op16;
-    __half* b16 = f16 ? a16 + M * K : nullptr;
-    if (f16)
-        if (int e = fill_f16_operands(g, !g_transposed, x, true, M, N, K, a16, b16, st)) return e;
-    auto launch = [&]() { return f16 ? launch_f16ops(a16, b16, p, st) : (g_transposed ? launch_dgrad_layout(g, x, p, st) : launch_wgrad_layout(g, x, p, st)); };
+    (void)op16; (void)op16_bytes;
+    auto launch = [&]() { return g_transposed ? launch_dgrad_layout(g, x, p, st) : launch_wgrad_layout(g, x, p, st); };
     if (splits == 1) {
         if (out_dtype == JF_F16) { p.mode = MODE_F16; p.out16 = (__half*)dw; }
         else { p.mode = MODE_F32; p.out32 = (float*)dw; }

@@ -1,319 +1,289 @@
 // The persistent per-block INT8 GEMM kernel (included by gemm.cu inside namespace jf, after the helpers it uses).
 //
-// Warp roles (19 warps): 16 consumer warps, 1 TMA producer warp, 2 MMA-issuing warps (one lane each).
+// What bounds it.  Every 128 x 128 x 32 block product (64 clocks on the tensor core) leaves tensor memory as 16384 int32 values that the
+// CUDA cores owe a conversion and a scale FMA each: 512 warp conversions on the ALU pipe (2 clocks each: 256 SM clocks) and 256
+// fma.rn.f32x2 on the FMA pipe (144 clocks).  The kernel needs ~440 SM clocks per block product (ALU pipe 69 % busy, issue slots 65 %).
 //
-// Hand-over of the accumulators.  Tensor memory holds two GROUPS of two 128-column accumulators.  The four K blocks of a
-// shared-memory stage form two pairs; pair 0 goes to group 0 and is issued by issuer 0, pair 1 to group 1 / issuer 1, each pair
-// is signalled with ONE tcgen05.commit.  Two issuers because the cost of issuing is the issuing thread's, not the tensor pipe's:
-// measured on B200 with a single-CTA microbenchmark, a thread that loops over [tcgen05.mma ; tcgen05.commit] needs ~457 SM clocks
-// per iteration whatever the MMA's N (16..256), ~110 more per additional MMA before the commit -- and two such threads in
-// different warps run at that rate EACH.  The shared-memory stage is released by a consumer warp once it has seen the stage's
-// last pair complete, which saves the issuers a third commit per stage.
+// Two CTAs share an SM.  One CTA of 16 consumer warps per SM moves in step: all its warps leave the same barrier, load the same
+// accumulator and then queue for the same pipe, and nothing computes during an epilogue.  Two independent CTAs of 128 x 64 tiles with
+// eight consumer warps each fill one another's gaps: 12288 x 3072 x 768 forward 131 -> 111 us (520 TOPS), both gradients of 7392 x 1600 x 1600 227 -> 154 us.
+// Their operand traffic (12 KB per block product and SM; TMA delivers 56 B per clock and SM from L2) stays below the arithmetic.
+// Copying the operands to fp16 first (kind::f16 delivers floats, no conversion) is no way around it: at 16 KB per block product the
+// loads alone take 290 clocks, and the copies cost as much as they save at the layer shapes; at 8192^3 that kernel drew 1725 MHz from the
+// power cap against 1920 MHz here and the two took the same time (1.55-1.60 ms).
 //
-// Consumers.  Warp w owns TMEM lanes 32*(w%4).. (rows) and columns 32*(w/4).. of every accumulator: a thread is one row of one
-// 32x32 quantisation block (32 fp32 accumulators in registers).  Every consumer warp has to walk through every K block, so the
-// length of one warp's chain per pair (barrier test, fences, two tcgen05.ld round trips, release, 2 x 48 arithmetic
-// instructions under four-way issue contention) is what bounds the kernel, not the tensor core (64 clocks per K block), the
-// issuers or the operand stream.
+// Warp roles (10 warps): 8 consumers, 1 TMA producer, 1 MMA issuer, each of the latter two with one elected lane (elect.sync: with
+// `lane == 0` instead, every tcgen05.mma and commit costs its thread ~100 clocks more).
 //
-// Abort path.  Every wait is bounded; when one expires the CTA's roles leave their loops.  Before the CTA frees its tensor
-// memory the producer waits (bounded) for the bulk copies it has in flight and each issuer commits its outstanding MMAs to a
-// scratch barrier and waits (bounded) for it, so that nothing writes into shared or tensor memory of an exited CTA.
+// Hand-over.  Tensor memory (256 columns per CTA) holds four 64-column accumulators in two PAIRS; K blocks 0, 1 of a stage go to pair 0,
+// K blocks 2, 3 to pair 1, one tcgen05.commit each.  One barrier wait and one arrival per warp serve two K blocks: the number of
+// instructions around the arithmetic is what the consumers' time depends on.  A short last stage passes its second pair on empty, so
+// that every tile starts at pair 0 and the consumers' loop has no branch and no register that names a slot.
+//
+// Consumers.  Warp w owns TMEM lanes 32*(w%4).. (rows) and columns 32*(w/4).. of every accumulator: a thread is one row of one 32x32
+// quantisation block (32 fp32 accumulators).  The scale products sa*sb of 32 K blocks sit one per lane and are broadcast by shuffle.
+//
+// Abort path.  Every wait is bounded; when one expires the CTA's flag is raised, the producer and the issuer leave their loops, the
+// consumers run through theirs without waiting.  Before the CTA frees its tensor memory the producer waits (bounded) for the bulk copies
+// it has in flight and the issuer commits its outstanding MMAs to a scratch barrier and waits (bounded) for it.
 #pragma once
 
-// Tile rasterisation: tiles are numbered in groups of RASTER_GM tile-rows, M-fastest inside a group, so the ~148 tiles that
-// are in flight together cover about 16 x 9 tiles: 16 A panels + 9 B panels (~26 MB at K = 8192) instead of a whole
-// 64-row-panel column of A, which did not stay in L2 (ncu: 1.12 GB of DRAM traffic per 8192^3 launch against 0.2 GB algorithmic).
+// Tiles are numbered in groups of RASTER_GM tile rows, M-fastest inside a group, so that the CTAs in flight together share A and B
+// panels that stay in L2.  (32-bit arithmetic: the launcher refuses problems with 2^31 tiles or more.)
 constexpr int RASTER_GM = 16;
-constexpr int EPI_WARPS = 16;                      // consumer warps
-constexpr int NUM_ISSUERS = 2;                     // MMA-issuing warps = accumulator groups
-constexpr int GEMM_THREADS = (EPI_WARPS + 1 + NUM_ISSUERS) * 32;
-// (32-bit arithmetic: the launcher refuses problems with 2^31 tiles or more, and 64-bit divisions cost ~40 instructions each)
-__device__ __forceinline__ void tile_coords(int64_t tile, int64_t tiles_m, int64_t tiles_n, int64_t& tm, int64_t& tn) {
-    const uint32_t t = (uint32_t)tile, tmx = (uint32_t)tiles_m, tnx = (uint32_t)tiles_n;
-    const uint32_t group_size = RASTER_GM * tnx;
-    const uint32_t group = t / group_size, in_group = t % group_size;
+__device__ __forceinline__ void tile_coords(uint32_t tile, uint32_t tiles_m, uint32_t tiles_n, int& tm, int& tn) {
+    const uint32_t group_size = RASTER_GM * tiles_n;
+    const uint32_t group = tile / group_size, in_group = tile % group_size;
     const uint32_t first_m = group * RASTER_GM;
-    const uint32_t gm = min((uint32_t)RASTER_GM, tmx - first_m);
-    tm = (int64_t)(first_m + in_group % gm);
-    tn = (int64_t)(in_group / gm);
+    const uint32_t gm = min((uint32_t)RASTER_GM, tiles_m - first_m);
+    tm = (int)(first_m + in_group % gm);
+    tn = (int)(in_group / gm);
+}
+
+// Wait for a barrier phase in as few instructions as the ready case allows (one try_wait and one branch).  A wait that outlasts the
+// clock budget, or that meets a raised abort flag, ends; the caller goes on (its results are void, every loop is finite).
+// OFF / ABORT_OFF: byte offsets of the barrier and of the abort flag from `base`.
+template <int OFF, int ABORT_OFF>
+__device__ __forceinline__ void tight_wait(uint32_t base, uint32_t parity) {
+    asm volatile(
+        "{\n\t.reg .pred P, Q;\n\t.reg .u32 t0, t1, f;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P, [%0+%2], %1;\n\t"
+        "@P bra DONE;\n\t"
+        "mov.u32 t0, %%clock;\n\t"
+        "LOOP:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P, [%0+%2], %1;\n\t"
+        "@P bra DONE;\n\t"
+        "ld.volatile.shared.u32 f, [%0+%3];\n\t"
+        "mov.u32 t1, %%clock;\n\t"
+        "sub.u32 t1, t1, t0;\n\t"
+        "setp.gt.u32 Q, t1, %4;\n\t"
+        "@Q st.volatile.shared.u32 [%0+%3], 4;\n\t"
+        "setp.ne.or.u32 Q, f, 0, Q;\n\t"
+        "@!Q bra LOOP;\n\t"
+        "DONE:\n\t}" ::"r"(base), "r"(parity), "n"(OFF), "n"(ABORT_OFF), "n"(WAIT_BUDGET_CLOCKS) : "memory");
+}
+// lane 0 arrives on the barrier at base + OFF
+template <int OFF>
+__device__ __forceinline__ void arrive_lane0(uint32_t base, int lane) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0+%2];\n\t}" ::"r"(base), "r"(lane), "n"(OFF) : "memory");
+}
+// The producer's and the issuer's wait: every try lets the hardware park the thread for up to 2 us.  False when it expired.
+__device__ __forceinline__ bool lean_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
+    if (__builtin_expect(ptx::mbar_try_wait_hint(bar, parity, 2000u), 1)) return true;
+    const uint32_t t0 = (uint32_t)clock();
+    while (!ptx::mbar_try_wait_hint(bar, parity, 2000u)) {
+        if (__builtin_expect(*abort_flag != 0, 0)) return false;
+        if (__builtin_expect((uint32_t)clock() - t0 > WAIT_BUDGET_CLOCKS, 0)) {
+            *abort_flag = code;
+            return false;
+        }
+    }
+    return true;
 }
 
 template <bool A_MN, bool B_MN, int CONV>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
+__global__ void __launch_bounds__(GEMM_THREADS, 2)
 gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
-    constexpr int WARP_TMA = EPI_WARPS, WARP_MMA = EPI_WARPS + 1;   // issuers: WARP_MMA, WARP_MMA + 1
-    constexpr bool INT32ACC = (CONV == CONV_INT32);
-    // F16OPS: the operands are fp16 copies of the int8 payloads (exact) and the MMAs are kind::f16 with fp32 accumulation, so
-    // the accumulator already holds float(I_p) (|I_p| < 2^20: every partial sum is an integer below 2^24, exact in fp32) and the
-    // consumers skip the int32 -> fp32 conversion.  A K block is 64 bytes of K instead of 32: a stage holds two 128 x 128 B
-    // boxes per operand (K blocks 0-1 and 2-3) and there are three stages; a K block is two K = 16 MMAs.
-    constexpr bool F16OPS = (CONV == CONV_F16OPS);
-    constexpr int NST = F16OPS ? 3 : STAGES;                            // pipeline stages
-    constexpr int OPER_STAGE = F16OPS ? 2 * STAGE_BYTES : STAGE_BYTES;  // bytes of one operand per stage
-    constexpr int NUM_GRP = NUM_ISSUERS, GRP_COLS = 2 * BN;   // two groups of two 128-column accumulators = all 512 TMEM columns
-    static_assert(NUM_GRP * GRP_COLS == TMEM_COLS && KB_PER_STAGE == 2 * NUM_GRP, "a stage = one pair of K blocks per group");
-
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* smem_a = smem;
-    uint8_t* smem_b = smem + NST * OPER_STAGE;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * NST * OPER_STAGE);
-    uint64_t* full_bar = bars;                            // [STAGES]   TMA -> MMA
-    uint64_t* empty_bar = bars + NST;                  // [STAGES]   consumers (int32 mode: MMA) -> TMA
-    uint64_t* grp_full = bars + 2 * NST;               // [NUM_GRP]  MMA -> consumers
-    uint64_t* grp_empty = bars + 2 * NST + NUM_GRP;    // [NUM_GRP]  consumers -> MMA
-    uint64_t* drain_bar = bars + 2 * NST + 2 * NUM_GRP;  // [NUM_ISSUERS]  abort path only: outstanding MMAs of an issuer
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * NST + 2 * NUM_GRP + NUM_ISSUERS);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    // barriers: pair_full[2] at 0, pair_empty[2] at 16, abort flag at 32, tmem slot at 36, drain at 40, full[STAGES] at 48,
+    // empty[STAGES] after them
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+    uint64_t* pair_full = bars;
+    uint64_t* pair_empty = bars + 2;
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 4);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4) + 1;
+    uint64_t* drain_bar = bars + 5;
+    uint64_t* full_bar = bars + 6;
+    uint64_t* empty_bar = full_bar + STAGES;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < NST; ++s) { ptx::mbar_init(&full_bar[s], 1); ptx::mbar_init(&empty_bar[s], 1); }
-        for (int g = 0; g < NUM_GRP; ++g) { ptx::mbar_init(&grp_full[g], 1); ptx::mbar_init(&grp_empty[g], EPI_WARPS); }
-        for (int g = 0; g < NUM_ISSUERS; ++g) ptx::mbar_init(&drain_bar[g], 1);
+        for (int s = 0; s < STAGES; ++s) { ptx::mbar_init(&full_bar[s], 1); ptx::mbar_init(&empty_bar[s], 1); }
+        for (int g = 0; g < 2; ++g) { ptx::mbar_init(&pair_full[g], 1); ptx::mbar_init(&pair_empty[g], CONSUMER_WARPS); }
+        ptx::mbar_init(drain_bar, 1);
         *abort_flag = 0;
         ptx::fence_barrier_init();
     }
-    if (warp == WARP_MMA) {
+    if (warp == CONSUMER_WARPS + 1) {
         ptx::tmem_alloc(tmem_slot, TMEM_COLS);
         ptx::tmem_relinquish();
-    }
-    if (warp == WARP_TMA && lane == 0) {
-        ptx::prefetch_tensormap(&map_a);
-        ptx::prefetch_tensormap(&map_b);
     }
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    const uint32_t num_tiles = (uint32_t)(p.tiles_m * p.tiles_n), num_items = num_tiles * (uint32_t)p.splits;
+    const int nkb = (int)p.nkb, per = (int)p.kb_per_split;
 
-    const int64_t num_tiles = p.tiles_m * p.tiles_n;
-    const int64_t num_items = num_tiles * p.splits;
-
-    if (warp == WARP_TMA) {
+    if (warp == CONSUMER_WARPS) {
         // ------------------------------------------------------------------ producer
-        if (lane == 0) {
-            uint32_t it = 0;   // running stage counter
+        if (ptx::elect_one()) {
+            uint32_t it = 0, s = 0, ph = 0;
             bool ok = true;
-            for (int64_t item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-                const int64_t tile = item % num_tiles, split = item / num_tiles;
-                int64_t tm, tn;
-                tile_coords(tile, p.tiles_m, p.tiles_n, tm, tn);
-                const int64_t kb0 = split * p.kb_per_split;
-                const int64_t kb1 = min(p.nkb, kb0 + p.kb_per_split);
-                for (int64_t kb = kb0; kb < kb1; kb += KB_PER_STAGE, ++it) {
-                    const uint32_t s = it % NST, ph = (it / NST) & 1u;
-                    if (!(ok = bounded_wait<true>(&empty_bar[s], ph ^ 1u, abort_flag, 1))) break;
-                    ptx::mbar_arrive_expect_tx(&full_bar[s], 2 * OPER_STAGE);
-                    const int32_t k_off = (int32_t)(kb * QB);
-                    if (F16OPS) {
-                        // K-major fp16 operands: two boxes of 64 elements of K each (the second one may lie past K: zero fill)
-                        ptx::tma_load_2d(smem_a + s * OPER_STAGE, &map_a, &full_bar[s], k_off, (int32_t)(tm * BM));
-                        ptx::tma_load_2d(smem_a + s * OPER_STAGE + STAGE_BYTES, &map_a, &full_bar[s], k_off + 64, (int32_t)(tm * BM));
-                        ptx::tma_load_2d(smem_b + s * OPER_STAGE, &map_b, &full_bar[s], k_off, (int32_t)(tn * BN));
-                        ptx::tma_load_2d(smem_b + s * OPER_STAGE + STAGE_BYTES, &map_b, &full_bar[s], k_off + 64, (int32_t)(tn * BN));
-                        continue;
-                    }
-                    if (A_MN) ptx::tma_load_2d(smem_a + s * STAGE_BYTES, &map_a, &full_bar[s], (int32_t)(tm * BM), k_off);
-                    else      ptx::tma_load_2d(smem_a + s * STAGE_BYTES, &map_a, &full_bar[s], k_off, (int32_t)(tm * BM));
-                    if (B_MN) ptx::tma_load_2d(smem_b + s * STAGE_BYTES, &map_b, &full_bar[s], (int32_t)(tn * BN), k_off);
-                    else      ptx::tma_load_2d(smem_b + s * STAGE_BYTES, &map_b, &full_bar[s], k_off, (int32_t)(tn * BN));
+            for (uint32_t item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+                const uint32_t tile = item % num_tiles, split = item / num_tiles;
+                int tm, tn;
+                tile_coords(tile, (uint32_t)p.tiles_m, (uint32_t)p.tiles_n, tm, tn);
+                const int kb0 = (int)split * per, kb1 = min(nkb, kb0 + per);
+                const int row = tm * BM, col = tn * BN;
+                for (int kb = kb0; kb < kb1; kb += KB_PER_STAGE) {
+                    if (!(ok = lean_wait(&empty_bar[s], ph ^ 1u, abort_flag, 1))) break;
+                    ptx::mbar_arrive_expect_tx(&full_bar[s], STAGE_BYTES);
+                    uint8_t* a = smem + s * STAGE_BYTES;
+                    const int k = kb * QB;
+                    ptx::tma_load_2d(a, &map_a, &full_bar[s], A_MN ? row : k, A_MN ? k : row);
+                    ptx::tma_load_2d(a + A_BYTES, &map_b, &full_bar[s], B_MN ? col : k, B_MN ? k : col);
+                    ++it;
+                    if (++s == STAGES) { s = 0; ph ^= 1u; }
                 }
             }
-            if (*abort_flag) {
-                // abort: the copies of the last (up to STAGES) armed stages may still be landing in this CTA's shared memory
-                for (uint32_t j = it > NST ? it - NST : 0u; j < it; ++j) drain_wait(&full_bar[j % NST], (j / NST) & 1u);
+            if (*abort_flag)
+                for (uint32_t j = it > STAGES ? it - STAGES : 0u; j < it; ++j) drain_wait(&full_bar[j % STAGES], (j / STAGES) & 1u);
+        }
+    } else if (warp == CONSUMER_WARPS + 1) {
+        // ------------------------------------------------------------------ MMA issuer
+        constexpr uint32_t idesc = ptx::make_idesc_i8(BM, BN, A_MN, B_MN);
+        uint32_t s = 0, ph = 0, par = 1;
+        bool ok = true;
+        const uint64_t da_base = ptx::make_smem_desc_sw128(ptx::smem_u32(smem), A_MN ? 128 * 128 : 16, 1024);
+        const uint64_t db_base = B_MN ? ptx::make_smem_desc_sw64(ptx::smem_u32(smem + A_BYTES), 128 * 64, 512)
+                                      : ptx::make_smem_desc_sw128(ptx::smem_u32(smem + A_BYTES), 16, 1024);
+        for (uint32_t item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+            const uint32_t split = item / num_tiles;
+            const int kb0 = (int)split * per, kb1 = min(nkb, kb0 + per);
+            for (int kb = kb0; kb < kb1 && ok; kb += KB_PER_STAGE) {
+                if (!(ok = __all_sync(0xffffffffu, lean_wait(&full_bar[s], ph, abort_flag, 2)))) break;
+                ptx::tc_fence_after();
+                const uint64_t da = da_base + (uint64_t)(s * (STAGE_BYTES / 16)), db = db_base + (uint64_t)(s * (STAGE_BYTES / 16));
+                const int nblk = min(KB_PER_STAGE, kb1 - kb);
+#pragma unroll
+                for (int pp = 0; pp < 2; ++pp) {
+                    if (!(ok = __all_sync(0xffffffffu, lean_wait(&pair_empty[pp], par, abort_flag, 3)))) break;
+                    ptx::tc_fence_after();
+                    if (ptx::elect_one()) {
+#pragma unroll
+                        for (int j = 2 * pp; j < 2 * pp + 2; ++j)
+                            if (j < nblk)
+                                ptx::umma_i8(tmem_base + j * BN, da + (uint64_t)(A_MN ? j * 256 : j * 2),
+                                             db + (uint64_t)(B_MN ? j * 128 : j * 2), idesc, 0u);
+                        ptx::umma_commit(&pair_full[pp]);       // a pair without a K block is passed on empty: every tile starts at pair 0
+                        if (pp == 1) ptx::umma_commit(&empty_bar[s]);
+                    }
+                    __syncwarp();
+                }
+                par ^= 1u;
+                if (++s == STAGES) { s = 0; ph ^= 1u; }
             }
         }
-    } else if (warp >= WARP_MMA) {
-        // ------------------------------------------------------------------ MMA issuers
-        const uint32_t w = (uint32_t)(warp - WARP_MMA);   // issuer index = accumulator group it owns
-        if (lane == 0 && !(INT32ACC && w != 0)) {
-            constexpr uint32_t idesc = ptx::make_idesc_i8(BM, BN, A_MN, B_MN);
-            uint32_t it = 0, gi = 0;   // running stage counter / uses of the accumulator group (int32 mode: tile counter)
-            bool ok = true;
-            for (int64_t item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-                const int64_t split = item / num_tiles;
-                const int64_t kb0 = split * p.kb_per_split;
-                const int64_t kb1 = min(p.nkb, kb0 + p.kb_per_split);
-                for (int64_t kb = kb0; kb < kb1 && ok; kb += KB_PER_STAGE, ++it) {
-                    const uint32_t s = it % NST, ph = (it / NST) & 1u;
-                    const int nblk = (int)min((int64_t)KB_PER_STAGE, kb1 - kb);
-                    if (!INT32ACC && nblk <= 2 * (int)w) continue;   // the stage holds no K block of this issuer's pair
-                    if (!(ok = bounded_wait<true>(&full_bar[s], ph, abort_flag, 2))) break;
-                    ptx::tc_fence_after();
-                    // descriptors of K block 0 of the stage; K block j is 32 bytes further along a K-major row and 32 K-rows
-                    // (4096 B) further in an MN-major tile, i.e. +2 / +256 in the descriptor's 16-byte address units
-                    const uint64_t da0 = ptx::make_smem_desc_sw128(ptx::smem_u32(smem_a + s * OPER_STAGE), A_MN ? 128 * 128 : 16, 1024);
-                    const uint64_t db0 = ptx::make_smem_desc_sw128(ptx::smem_u32(smem_b + s * OPER_STAGE), B_MN ? 128 * 128 : 16, 1024);
-                    if (INT32ACC) {
-                        // diagnostic mode: one issuer; the tensor core accumulates the whole K range of a tile in one accumulator
-                        const uint32_t g = gi % NUM_GRP;
-                        for (int j = 0; j < nblk && ok; ++j) {
-                            const bool first = (kb + j == kb0), last = (kb + j + 1 == kb1);
-                            if (first) {
-                                if (!(ok = bounded_wait<true>(&grp_empty[g], ((gi / NUM_GRP) & 1u) ^ 1u, abort_flag, 3))) break;
-                                ptx::tc_fence_after();
-                            }
-                            ptx::umma_i8(tmem_base + g * GRP_COLS, da0 + (uint64_t)(A_MN ? j * 256 : j * 2),
-                                         db0 + (uint64_t)(B_MN ? j * 256 : j * 2), idesc, first ? 0u : 1u);
-                            if (last) { ptx::umma_commit(&grp_full[g]); ++gi; }
-                        }
-                        if (ok) ptx::umma_commit(&empty_bar[s]);   // no consumer sees the stages of this mode: the issuer frees them
-                    } else {
-                        if (!(ok = bounded_wait<true>(&grp_empty[w], (gi & 1u) ^ 1u, abort_flag, 3))) break;
-                        ptx::tc_fence_after();
-                        const int npair = min(2, nblk - 2 * (int)w);
-                        for (int jj = 0; jj < npair; ++jj) {
-                            const int j = 2 * (int)w + jj;
-                            if (F16OPS) {
-                                // issuer w's pair lives in box w of the stage; K block jj of the pair starts 64 B into the 128-byte
-                                // swizzle row, its two K = 16 halves are 32 B apart (descriptor address units of 16 B)
-                                constexpr uint32_t idesc16 = ptx::make_idesc_f16(BM, BN);
-                                const uint64_t off = (uint64_t)(w * (STAGE_BYTES / 16) + jj * 4);
-                                ptx::umma_f16(tmem_base + w * GRP_COLS + jj * BN, da0 + off, db0 + off, idesc16, 0u);
-                                ptx::umma_f16(tmem_base + w * GRP_COLS + jj * BN, da0 + off + 2, db0 + off + 2, idesc16, 1u);
-                                continue;
-                            }
-                            ptx::umma_i8(tmem_base + w * GRP_COLS + jj * BN, da0 + (uint64_t)(A_MN ? j * 256 : j * 2),
-                                         db0 + (uint64_t)(B_MN ? j * 256 : j * 2), idesc, 0u);
-                        }
-                        ptx::umma_commit(&grp_full[w]);
-                        ++gi;
-                    }
-                }
-            }
-            if (*abort_flag) {
-                // abort: wait until every MMA this thread has issued has completed (they read shared and write tensor memory)
-                ptx::umma_commit(&drain_bar[w]);
-                drain_wait(&drain_bar[w], 0u);
-            }
+        if (*abort_flag && ptx::elect_one()) {
+            ptx::umma_commit(drain_bar);
+            drain_wait(drain_bar, 0u);
         }
     } else {
         // ------------------------------------------------------------------ consumers
-        const int quad = warp & 3, cgrp = warp >> 2;   // TMEM lane quadrant (rows) / 32-column group of every accumulator
-        uint32_t use0 = 0, use1 = 0, sit = 0;   // uses of group 0 / 1 (int32 mode: use0 counts tiles) / running stage counter
-        bool ok = true;
-        const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16) + cgrp * 32;
-        for (int64_t item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-            int tm32, tn32, split32;
-            {
-                const uint32_t tile = (uint32_t)item % (uint32_t)num_tiles;
-                int64_t tm, tn;
-                tile_coords(tile, p.tiles_m, p.tiles_n, tm, tn);
-                tm32 = (int)tm; tn32 = (int)tn; split32 = (int)((uint32_t)item / (uint32_t)num_tiles);
-            }
-            const int kb0 = (int)(split32 * p.kb_per_split);
-            const int kb1 = (int)min(p.nkb, (int64_t)kb0 + p.kb_per_split);
-            const int rowblk = tm32 * (BM / QB) + quad;
-            const int colblk = tn32 * (BN / QB) + cgrp;
+        const int quad = warp & 3, cg = warp >> 2;
+        const uint32_t base = ptx::smem_u32(bars);
+        const uint32_t t0 = tmem_base + ((uint32_t)(quad * 32) << 16) + cg * 32;
+        uint32_t par = 0;
+        for (uint32_t item = blockIdx.x; item < num_items; item += gridDim.x) {
+            const uint32_t tile = item % num_tiles, split = item / num_tiles;
+            int tm, tn;
+            tile_coords(tile, (uint32_t)p.tiles_m, (uint32_t)p.tiles_n, tm, tn);
+            const int kb0 = (int)split * per, n = min(nkb, kb0 + per) - kb0;
+            const int rowblk = tm * (BM / QB) + quad, colblk = tn * (BN / QB) + cg;
             const bool blk_ok = rowblk < (int)(p.M / QB) && colblk < (int)(p.N / QB);   // warp-uniform
 
-            uint64_t acc2[16];   // the thread's 32 fp32 accumulators as packed pairs
+            uint64_t acc[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) acc2[j] = 0ull;
-            auto accumulate = [&](const uint32_t (&raw)[32], float sc) { scale_accumulate<CONV>(acc2, raw, sc); };
-
-            // lanes 0-7 hold the scale products sa*sb of 8 consecutive K blocks
-            const __half* sa_ptr = p.sa + (int64_t)rowblk * p.sa_sm + (int64_t)(kb0 + (lane & 7)) * p.sa_sk;
-            const __half* sb_ptr = p.sb + (int64_t)colblk * p.sb_sn + (int64_t)(kb0 + (lane & 7)) * p.sb_sk;
-            // The two loads are volatile asm so that they are ISSUED here, eight K blocks before their values are needed (a plain
-            // __ldg is sunk by the compiler to its first use, which exposed the load latency once per eight K blocks).
-            auto fetch_scales = [&](int t8) -> float {   // t8 = first K block (relative to kb0) of the group of 8
-                unsigned short ha = 0, hb = 0;
-                if (lane < 8 && kb0 + t8 + (lane & 7) < kb1 && blk_ok) {
-                    asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(ha) : "l"(sa_ptr + (int64_t)t8 * p.sa_sk));
-                    asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(hb) : "l"(sb_ptr + (int64_t)t8 * p.sb_sk));
+            for (int j = 0; j < 16; ++j) acc[j] = 0ull;
+            // lane l holds the scale product of K block 32 i + l
+            const __half* sa_ptr = p.sa + (int64_t)rowblk * p.sa_sm + (int64_t)(kb0 + lane) * p.sa_sk;
+            const __half* sb_ptr = p.sb + (int64_t)colblk * p.sb_sn + (int64_t)(kb0 + lane) * p.sb_sk;
+            unsigned short ha = 0, hb = 0;
+            auto fetch_scales = [&](int t) {
+                if (CONV != CONV_INT32 && t + lane < n && blk_ok) {
+                    asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(ha) : "l"(sa_ptr + (int64_t)t * p.sa_sk));
+                    asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(hb) : "l"(sb_ptr + (int64_t)t * p.sb_sk));
                 }
-                return __fmul_rn(__half2float(__ushort_as_half(ha)), __half2float(__ushort_as_half(hb)));
             };
-            float sc_next = INT32ACC ? 0.f : fetch_scales(0);
-            float sc_cur = 0.f;
-            const int nloop = INT32ACC ? (kb1 > kb0 ? 1 : 0) : (kb1 - kb0);   // the int32 mode reads one accumulated tile
-            const uint32_t g32 = use0 % NUM_GRP;                               // int32 mode: the tile's group
-
-            // One pair of K blocks (group g; `two` = the pair has its second K block; `stage_end` = last pair of its shared-memory
-            // stage).  Returns false when a wait expired.
-            // Registers (96 per thread with 19 warps) hold 32 accumulators + ONE accumulator's 32 raw columns: the pair's first
-            // K block is converted and accumulated before the second one is read, and only then can the group be released.
-            // Reading both first and releasing at once would shorten the hand-over (measured without arithmetic: 1.26 ms
-            // instead of 1.43 ms at 8192^3) but needs 64 raw registers, and the spills cost far more than that.
-            auto do_pair = [&](const uint32_t g, const bool two, const float s0, const float s1, const bool stage_end) -> bool {
-                const uint32_t acc = lane_base + g * GRP_COLS;
-                {
-                    const uint32_t uses = INT32ACC ? use0 / NUM_GRP : (g ? use1 : use0);
-                    const bool got = bounded_wait(&grp_full[g], uses & 1u, abort_flag, 4);
-                    if (!__all_sync(0xffffffffu, got)) return false;   // warp-uniform exit
-                    if (g && !INT32ACC) ++use1; else ++use0;
-                    ptx::tc_fence_after();
-                }
-                uint32_t r[32];
-                ptx::tmem_ld_32x32b_x32(acc, r);
-                ptx::tmem_wait_ld_regs(r);
-                if (two) {
-                    accumulate(r, s0);
-                    ptx::tmem_ld_32x32b_x32(acc + BN, r);
-                    ptx::tmem_wait_ld_regs(r);
-                }
-                // the group's accumulators have left tensor memory: hand the group back to its issuer
-                ptx::tc_fence_before();
+            fetch_scales(0);
+            float sc = 0.f;
+            auto pair = [&](auto pp_c, int k, int left) {          // `left` K blocks remain (the pair holds min(2, left) of them)
+                constexpr int PP = decltype(pp_c)::value;
+                const float s0 = __shfl_sync(0xffffffffu, sc, k), s1 = __shfl_sync(0xffffffffu, sc, k + 1);
+                tight_wait<8 * PP, 32>(base, par);
                 __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(&grp_empty[g]);
-                if (!INT32ACC && stage_end) {
-                    // the last pair of a shared-memory stage has completed (the earlier pair was seen before): hand the stage
-                    // back to the TMA producer
-                    if (warp == 0 && lane == 0) ptx::mbar_arrive(&empty_bar[sit % NST]);
-                    ++sit;
-                }
-                accumulate(r, two ? s1 : s0);
-                return true;
-            };
-
-            int t = 0;
-            if (!INT32ACC) {
-                // fast path: eight K blocks (two stages, groups 0 1 0 1) per iteration with everything about the pair a constant
-                for (; t + 8 <= nloop && ok; t += 8) {
-                    sc_cur = sc_next;
-                    sc_next = fetch_scales(t + 8);
-#pragma unroll
-                    for (int pp = 0; pp < 4; ++pp) {
-                        if (!ok) break;
-                        ok = do_pair((uint32_t)(pp & 1), true, __shfl_sync(0xffffffffu, sc_cur, 2 * pp),
-                                     __shfl_sync(0xffffffffu, sc_cur, 2 * pp + 1), (pp & 1) == 1);
+                ptx::tc_fence_after();
+                uint32_t r[32];
+                if (left > 1) {
+                    ptx::tmem_ld_wait_32x32b_x32(t0 + 128 * PP, r);
+                    scale_accumulate<CONV>(acc, r, s0);
+                    ptx::tmem_ld_wait_32x32b_x32(t0 + 128 * PP + 64, r);
+                    ptx::tc_fence_before();
+                    arrive_lane0<16 + 8 * PP>(base, lane);
+                    scale_accumulate<CONV>(acc, r, s1);
+                } else {
+                    if (left == 1) {
+                        ptx::tmem_ld_wait_32x32b_x32(t0 + 128 * PP, r);
+                        scale_accumulate<CONV>(acc, r, s0);
                     }
+                    ptx::tc_fence_before();
+                    arrive_lane0<16 + 8 * PP>(base, lane);
                 }
-            }
-            for (; t < nloop && ok; t += 2) {
-                // remaining pairs: pair t/2 of the tile lives in group (t/2)%2 (the int32 mode: one accumulator per tile)
-                const uint32_t g = INT32ACC ? g32 : (uint32_t)((t >> 1) & 1);
-                const int pi = (int)(t & 7);
-                if (!INT32ACC && pi == 0) {
-                    sc_cur = sc_next;
-                    sc_next = fetch_scales(t + 8);
+            };
+            using I0 = std::integral_constant<int, 0>; using I1 = std::integral_constant<int, 1>;
+// eight K blocks (both pairs twice) without a branch
+            auto full_pair = [&](auto pp_c, float s0, float s1) {
+                constexpr int PP = decltype(pp_c)::value;
+                tight_wait<8 * PP, 32>(base, par);
+                __syncwarp();
+                ptx::tc_fence_after();
+                uint32_t r[32];
+                ptx::tmem_ld_wait_32x32b_x32(t0 + 128 * PP, r);
+                scale_accumulate<CONV>(acc, r, s0);
+                ptx::tmem_ld_wait_32x32b_x32(t0 + 128 * PP + 64, r);
+                ptx::tc_fence_before();
+                arrive_lane0<16 + 8 * PP>(base, lane);
+                scale_accumulate<CONV>(acc, r, s1);
+            };
+            int t = 0;
+#pragma unroll 1
+            for (; t + 8 <= n; t += 8) {
+                const int k = t & 31;
+                if (k == 0) {
+                    sc = __fmul_rn(__half2float(__ushort_as_half(ha)), __half2float(__ushort_as_half(hb)));
+                    fetch_scales(t + 32);
                 }
-                const float s0 = __shfl_sync(0xffffffffu, sc_cur, pi);
-                const float s1 = __shfl_sync(0xffffffffu, sc_cur, pi + 1);
-                ok = do_pair(g, t + 1 < nloop, s0, s1, g == 1 || t + 2 >= nloop);
-            }
-            if (!ok) break;
-
-            // ---------------------------------------------------------------- tile epilogue
-            if (!blk_ok) continue;
-            float ab[32];
+                const float sk = __shfl_sync(0xffffffffu, sc, k + (lane & 7));     // lane l: K block k + l % 8
 #pragma unroll
-            for (int j = 0; j < 16; ++j) unpack2(acc2[j], ab[2 * j], ab[2 * j + 1]);
-            store_block(p, ab, (int64_t)tm32 * BM + quad * 32 + lane, (int64_t)colblk * QB, rowblk, colblk, split32, lane);
+                for (int q = 0; q < 2; ++q) {
+                    full_pair(I0{}, __shfl_sync(0xffffffffu, sk, 4 * q), __shfl_sync(0xffffffffu, sk, 4 * q + 1));
+                    full_pair(I1{}, __shfl_sync(0xffffffffu, sk, 4 * q + 2), __shfl_sync(0xffffffffu, sk, 4 * q + 3));
+                    par ^= 1u;
+                }
+            }
+#pragma unroll 1
+            for (; t < n; t += 4) {
+                const int k = t & 31;
+                if (k == 0) {
+                    sc = __fmul_rn(__half2float(__ushort_as_half(ha)), __half2float(__ushort_as_half(hb)));
+                    fetch_scales(t + 32);
+                }
+                pair(I0{}, k, n - t);
+                pair(I1{}, k + 2, n - t - 2);
+                par ^= 1u;
+            }
+            if (!blk_ok) continue;
+            store_block(p, acc, (int64_t)rowblk * QB + lane, (int64_t)colblk * QB, rowblk, colblk, split, lane);
         }
     }
-
-    // ---------------------------------------------------------------------- teardown
     ptx::tc_fence_before();
     __syncthreads();
-    if (warp == WARP_MMA) {
-        __syncwarp();
+    if (threadIdx.x == 0 && *abort_flag) atomicCAS(&g_gemm_error, 0, *abort_flag);
+    if (warp == CONSUMER_WARPS + 1) {
         ptx::tc_fence_after();
         ptx::tmem_dealloc(tmem_base, TMEM_COLS);
     }
 }
+

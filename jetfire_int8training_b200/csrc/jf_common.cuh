@@ -139,6 +139,18 @@ __device__ __forceinline__ float byte_to_float(uint32_t wx, int k) {
     return __fadd_rn(__uint_as_float(__byte_perm(wx, 0x4B000000u, sel)), -8388736.0f);
 }
 
+// The noise of philox_noise8 as four packed pairs: both halves of a word are placed over the exponent of 2^23 and rescaled by one
+// two-wide FMA (the same bits as half_to_noise).
+__device__ __forceinline__ void philox_noise8x2(uint64_t e, const PhiloxKeys& keys, uint64_t offset, uint64_t (&out)[4]) {
+    const uint64_t g = e >> 3;
+    const uint4 w = philox4x32_10(make_uint4((uint32_t)g, (uint32_t)(g >> 32), (uint32_t)offset, (uint32_t)(offset >> 32)), keys);
+    const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
+    const uint64_t k2 = f2_pack(1.52587890625e-05f, 1.52587890625e-05f), c2 = f2_pack(-128.5f, -128.5f);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        out[j] = f2_fma(f2_pack(__uint_as_float(__byte_perm(ws[j], 0x4B000000u, 0x7410)), __uint_as_float(__byte_perm(ws[j], 0x4B000000u, 0x7432))), k2, c2);
+}
+
 // dtype-generic 16-element row chunk loads -> fp32
 template <typename T>
 struct Load16;

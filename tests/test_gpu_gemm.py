@@ -115,6 +115,25 @@ def test_backward_bit_exact(LIN, oracle, op16, M, N, K):
     assert_bits_equal(n(g16), do, "dgrad dequantised")
 
 
+@pytest.mark.parametrize("nkb", [1, 2, 3, 4, 5, 7, 8, 9, 31, 32, 33, 40])
+@pytest.mark.parametrize("M,N", [(32, 32), (160, 96)])
+def test_k_block_counts_and_tile_edges(LIN, oracle, M, N, nkb):
+    """K blocks around the kernel's stage (4), unrolled step (8) and scale fetch (32), on tiles with one and with several ragged edges,
+    in the three layouts (the weight gradient sums over nkb blocks too)."""
+    A, B, SA, SB = rand_operands(17 * nkb + M, M, N, 32 * nkb)
+    q, s = LIN.int8_linear_forward(t(A), t(SA), t(B), t(SB), True, 32)
+    qo, so = oracle.linear_forward(A, SA, B, SB)
+    assert_bits_equal(n(q), qo, "payload"); assert_bits_equal(n(s), so, "scales")
+    W, SW = np.ascontiguousarray(B.T), np.ascontiguousarray(SB.T)               # dgrad: dX = dY W with dY [M, K], W [K, N]
+    X, SX = rand_operands(nkb, M, N, 32)[0][:, :1].repeat(N, 1), np.full((M // 32, N // 32), 0.01, np.float16)
+    gx, gs, _ = LIN.int8_linear_backward(t(X), t(SX), t(A), t(SA), None, t(W), t(SW), 32, stochastic=False, wgrad_split_k=1)
+    qo, so = oracle.linear_dgrad(A, SA, W, SW, None)
+    assert_bits_equal(n(gx), qo, "dgrad payload"); assert_bits_equal(n(gs), so, "dgrad scales")
+    G, SG = np.ascontiguousarray(A.T), np.ascontiguousarray(SA.T)               # wgrad: dW = dY^T X with dY [K, M], X [K, N]
+    dw = LIN.int8_linear_wgrad(t(W), t(SW), t(G), t(SG), torch.float32, 1)
+    assert_bits_equal(n(dw), oracle.linear_wgrad(G, SG, W, SW, out_dtype=np.float32), "wgrad")
+
+
 @pytest.mark.parametrize("tokens,Cin,Cout,split", [(2048, 128, 128, 4), (4096, 768, 768, 0), (1024, 96, 160, 3)])
 def test_wgrad_split_k_is_deterministic_and_matches_oracle(LIN, L, oracle, op16, tokens, Cin, Cout, split):
     rng = np.random.default_rng(tokens + split)
