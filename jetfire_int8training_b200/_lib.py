@@ -1,4 +1,5 @@
-"""ctypes binding of the C ABI declared in include/jetfire_b200.h.
+"""Bindings of the C ABI declared in include/jetfire_b200.h: `lib()` is the library through ctypes (every entry point), `host()` the
+native module through which the operators call it (csrc/host_ops.cpp).
 
 There is no CPU fallback: if the compiled library is missing, importing an operator raises, and every
 operator raises on non-CUDA tensors.
@@ -8,6 +9,7 @@ import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libjetfire_b200.so")
+HOST_PATH = os.path.join(HERE, "_host_ops.so")
 
 _i64, _u64, _int, _vp = ctypes.c_int64, ctypes.c_uint64, ctypes.c_int, ctypes.c_void_p
 
@@ -45,6 +47,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_host = None
 
 
 class JetfireError(RuntimeError):
@@ -66,6 +69,23 @@ def lib():
             fn.restype = res
         _lib = L
     return _lib
+
+
+def host():
+    """The operators' native host path; raises if it has not been built."""
+    global _host
+    if _host is None:
+        lib()
+        if not os.path.exists(HOST_PATH):
+            raise JetfireError(f"{HOST_PATH} is missing: build it with `python -m jetfire_int8training_b200.build`")
+        import importlib.util
+        import torch  # noqa: F401  (its libraries have to be loaded first)
+        spec = importlib.util.spec_from_file_location("jetfire_int8training_b200._host_ops", HOST_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.set_error_class(JetfireError)
+        _host = module
+    return _host
 
 
 def check(status, what):
