@@ -73,6 +73,7 @@ __device__ __forceinline__ void drain_wait(uint64_t* bar, uint32_t parity) {
 // FMA pipe and a subtraction of 1.5*2^23 for 1/8, 1/4 or 1/2 of the values, to relieve the ALU pipe, measured 1-15 % slower.)
 // CONV_INT32 adds the raw integers instead: the plain int32 GEMM behind jf_igemm_int32.
 // ---------------------------------------------------------------------------------------------------------
+constexpr int NO_SR = -1;     // beside the values of Noise
 enum ConvMode : int { CONV_I2F = 0, CONV_INT32 = 1 };
 
 // acc2[j] (16 packed pairs) += s * float(r[2j], r[2j+1]) for the 32 int32 values in r
@@ -143,18 +144,18 @@ __device__ __forceinline__ void store_block(const GemmParams& p, const uint64_t 
         // only stochastic rounding can leave [-127, 127], so only it needs the clamp.
         const bool fast = __all_sync(0xffffffffu, d.fast || zero);
         auto quantise_all = [&](auto fast_c, auto sr_c, auto deq_c) {
-            constexpr bool FAST = decltype(fast_c)::value, SRND = decltype(sr_c)::value, DEQ = decltype(deq_c)::value;
+            constexpr bool FAST = decltype(fast_c)::value, SRND = decltype(sr_c)::value != NO_SR, DEQ = decltype(deq_c)::value;
             uint32_t words[8];
 #pragma unroll
             for (int k8 = 0; k8 < 4; ++k8) {      // 8 elements = one Philox call
                 uint64_t nz2[4] = {0ull, 0ull, 0ull, 0ull};
                 if (SRND) {
-                    if (p.noise) {
+                    if (decltype(sr_c)::value == NOISE_GIVEN) {
                         const float4 n0 = __ldg(reinterpret_cast<const float4*>(p.noise + row * p.N + col + 8 * k8));
                         const float4 n1 = __ldg(reinterpret_cast<const float4*>(p.noise + row * p.N + col + 8 * k8 + 4));
                         nz2[0] = f2_pack(n0.x, n0.y); nz2[1] = f2_pack(n0.z, n0.w); nz2[2] = f2_pack(n1.x, n1.y); nz2[3] = f2_pack(n1.z, n1.w);
                     } else {
-                        philox_noise8x2((uint64_t)(row * p.N + col + 8 * k8), p.keys, p.offset, nz2);
+                        philox_noise8x2<decltype(sr_c)::value == NOISE_PHILOX_WIDE>((uint64_t)(row * p.N + col + 8 * k8), p.keys, p.offset, nz2);
                     }
                 }
                 uint32_t bits[8], h16[4];
@@ -202,11 +203,21 @@ __device__ __forceinline__ void store_block(const GemmParams& p, const uint64_t 
             }
         };
         using T_ = std::true_type; using F_ = std::false_type;
-        auto rounding = [&](auto fast_c) {
-            if (p.mode == MODE_INT8) { if (p.stochastic) quantise_all(fast_c, T_{}, F_{}); else quantise_all(fast_c, F_{}, F_{}); }
-            else                     { if (p.stochastic) quantise_all(fast_c, T_{}, T_{}); else quantise_all(fast_c, F_{}, T_{}); }
+        auto rounding = [&](auto fast_c, auto sr_c) {
+            if (p.mode == MODE_INT8) quantise_all(fast_c, sr_c, F_{}); else quantise_all(fast_c, sr_c, T_{});
         };
-        if (fast) rounding(T_{}); else rounding(F_{});
+        if (!p.stochastic) {
+            using N_ = std::integral_constant<int, NO_SR>;
+            if (fast) rounding(T_{}, N_{}); else rounding(F_{}, N_{});
+        } else if (p.noise) {
+            using G_ = std::integral_constant<int, NOISE_GIVEN>;
+            if (fast) rounding(T_{}, G_{}); else rounding(F_{}, G_{});
+        } else if (fast && p.M < PHILOX_WIDE_ELEMENTS / p.N) {
+            rounding(T_{}, std::integral_constant<int, NOISE_PHILOX>{});
+        } else {
+            using W_ = std::integral_constant<int, NOISE_PHILOX_WIDE>;
+            if (fast) rounding(T_{}, W_{}); else rounding(F_{}, W_{});
+        }
     }
 }
 
@@ -367,7 +378,7 @@ int jf_igemm_dgrad(const int8_t* g, const int8_t* w, const void* sg, int64_t sg_
     p.M = M; p.N = N; p.K = K; p.splits = 1; p.kb_per_split = K / QB;
     p.sa = (const __half*)sg; p.sa_sm = sg_stride_m; p.sa_sk = sg_stride_k;
     p.sb = (const __half*)sw; p.sb_sn = sw_stride_n; p.sb_sk = sw_stride_k;
-    p.stochastic = stochastic; p.noise = noise; p.keys = make_philox_keys(seed); p.offset = offset;
+    p.stochastic = stochastic; p.noise = noise; p.keys = make_philox_keys(seed, offset); p.offset = offset;
     if (out_mode == JF_OUT_INT8) {
         if (!dx8 || !sdx) return JF_ERR_NULL;
         if (!aligned16(dx8)) return JF_ERR_ALIGN;

@@ -33,19 +33,19 @@ inline bool mult32(int64_t v) { return v > 0 && (v % 32) == 0; }
 // Noise mapping.  One Philox call (four 32-bit words) serves the 8 consecutive elements of group g = e / 8; element e uses the
 // 16-bit half (e & 1) of word (e >> 1) & 3:  noise = h * 2^-16 - 0.5, a multiple of 2^-16 in [-0.5, 0.5) like the reference's
 // uniform_(-0.5, 0.5).  Built without an int->float conversion: the half is placed in the low mantissa bits of 2^23, and one
-// FMA rescales it: (2^23 + h) * 2^-16 - 128.5 = h * 2^-16 - 0.5, exact in fp32.
-__device__ __forceinline__ float half_to_noise(uint32_t w, int hi) {
-    const uint32_t bits = __byte_perm(w, 0x4B000000u, hi ? 0x7432 : 0x7410);   // {h.lo, h.hi, 0x00, 0x4B}
-    return __fmaf_rn(__uint_as_float(bits), 1.52587890625e-05f, -128.5f);
-}
+// FMA rescales it: (2^23 + h) * 2^-16 - 128.5 = h * 2^-16 - 0.5, exact in fp32 (noise2 below).
 
-// The ten round keys of Philox4x32-10 for one seed (key schedule: k + r * (0x9E3779B9, 0xBB67AE85)), computed on the host and
-// passed with the kernel parameters: in the kernel they are constant-bank operands of the round's XOR, which saves the 18
-// additions of the schedule per call (a call serves only 8 elements, so the generator is a large part of every stochastic kernel).
+// What a call of Philox4x32-10 needs besides the group number: the ten round keys of the seed (key schedule: k + r * (0x9E3779B9,
+// 0xBB67AE85)), computed on the host and passed with the kernel parameters (constant-bank operands of the rounds' XORs), and the parts
+// of the first three rounds that do not depend on the low half of the group number.  With the counter (g_lo, 0, offset_lo, offset_hi)
+//   round 1: one product of g_lo; the product of offset_lo is a constant of the launch,
+//   round 2: x is such a constant too, so its product is, and round 3 sees one of its halves:
+// 18 multiplications instead of 20 per call of 8 elements.  Group numbers of 2^32 and more (2^35 elements) take all rounds.
 struct PhiloxKeys {
     uint32_t k[20];
+    uint32_t z1, x2, z2, z3;    // XOR constants: z of round 1, x and z of round 2, z of round 3
 };
-inline PhiloxKeys make_philox_keys(uint64_t seed) {
+inline PhiloxKeys make_philox_keys(uint64_t seed, uint64_t offset) {
     PhiloxKeys ks;
     uint32_t kx = (uint32_t)seed, ky = (uint32_t)(seed >> 32);
     for (int r = 0; r < 10; ++r) {
@@ -54,26 +54,35 @@ inline PhiloxKeys make_philox_keys(uint64_t seed) {
         kx += 0x9E3779B9u;
         ky += 0xBB67AE85u;
     }
+    const uint64_t p1 = 0xCD9E8D57ull * (uint32_t)offset;                       // round 1, product of z = offset_lo
+    const uint32_t x = (uint32_t)(p1 >> 32) ^ ks.k[0];                          // round 1: x' = hi ^ y (= 0) ^ key
+    const uint64_t p0 = 0xD2511F53ull * x;                                      // round 2, product of x
+    ks.z1 = (uint32_t)(offset >> 32) ^ ks.k[1];
+    ks.x2 = (uint32_t)p1 ^ ks.k[2];
+    ks.z2 = (uint32_t)(p0 >> 32) ^ ks.k[3];
+    ks.z3 = (uint32_t)p0 ^ ks.k[5];
     return ks;
 }
-__device__ __forceinline__ uint4 philox4x32_10(uint4 c, const PhiloxKeys& ks) {
+// (64-bit products: one wide multiply-add instruction yields both halves)
+__device__ __forceinline__ uint4 philox_rounds(uint4 c, const PhiloxKeys& ks, int first) {
 #pragma unroll
     for (int r = 0; r < 10; ++r) {
-        const uint32_t hi0 = __umulhi(0xD2511F53u, c.x), lo0 = 0xD2511F53u * c.x;
-        const uint32_t hi1 = __umulhi(0xCD9E8D57u, c.z), lo1 = 0xCD9E8D57u * c.z;
-        c = make_uint4(hi1 ^ c.y ^ ks.k[2 * r], lo1, hi0 ^ c.w ^ ks.k[2 * r + 1], lo0);
+        if (r < first) continue;
+        const uint64_t p0 = (uint64_t)0xD2511F53u * c.x, p1 = (uint64_t)0xCD9E8D57u * c.z;
+        c = make_uint4((uint32_t)(p1 >> 32) ^ c.y ^ ks.k[2 * r], (uint32_t)p1, (uint32_t)(p0 >> 32) ^ c.w ^ ks.k[2 * r + 1], (uint32_t)p0);
     }
     return c;
 }
-
-// Noise for the 8 consecutive elements starting at linear index e (e % 8 == 0).
-__device__ __forceinline__ void philox_noise8(uint64_t e, const PhiloxKeys& keys, uint64_t offset, float out[8]) {
-    const uint64_t g = e >> 3;
-    const uint4 w = philox4x32_10(make_uint4((uint32_t)g, (uint32_t)(g >> 32), (uint32_t)offset, (uint32_t)(offset >> 32)), keys);
-    out[0] = half_to_noise(w.x, 0); out[1] = half_to_noise(w.x, 1);
-    out[2] = half_to_noise(w.y, 0); out[3] = half_to_noise(w.y, 1);
-    out[4] = half_to_noise(w.z, 0); out[5] = half_to_noise(w.z, 1);
-    out[6] = half_to_noise(w.w, 0); out[7] = half_to_noise(w.w, 1);
+// WIDE: group numbers may need more than 32 bits.  A template parameter, chosen once per launch: a test inside would end the basic block,
+// and the scheduler could not interleave the serial chains of several calls (quantize + SR of [12288 x 2304]: 29.4 us with the test).
+template <bool WIDE>
+__device__ __forceinline__ uint4 philox_group(uint64_t g, const PhiloxKeys& ks, uint64_t offset) {
+    if (WIDE) return philox_rounds(make_uint4((uint32_t)g, (uint32_t)(g >> 32), (uint32_t)offset, (uint32_t)(offset >> 32)), ks, 0);
+    const uint64_t a = (uint64_t)0xD2511F53u * (uint32_t)g;                     // round 1
+    const uint64_t b = (uint64_t)0xCD9E8D57u * ((uint32_t)(a >> 32) ^ ks.z1);   // round 2
+    const uint32_t x = (uint32_t)(b >> 32) ^ ks.x2, z = (uint32_t)a ^ ks.z2;
+    const uint64_t p0 = (uint64_t)0xD2511F53u * x, p1 = (uint64_t)0xCD9E8D57u * z;   // round 3: y = lo of b, w = constant
+    return philox_rounds(make_uint4((uint32_t)(p1 >> 32) ^ (uint32_t)b ^ ks.k[4], (uint32_t)p1, (uint32_t)(p0 >> 32) ^ ks.z3, (uint32_t)p0), ks, 3);
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -139,17 +148,22 @@ __device__ __forceinline__ float byte_to_float(uint32_t wx, int k) {
     return __fadd_rn(__uint_as_float(__byte_perm(wx, 0x4B000000u, sel)), -8388736.0f);
 }
 
-// The noise of philox_noise8 as four packed pairs: both halves of a word are placed over the exponent of 2^23 and rescaled by one
-// two-wide FMA (the same bits as half_to_noise).
-__device__ __forceinline__ void philox_noise8x2(uint64_t e, const PhiloxKeys& keys, uint64_t offset, uint64_t (&out)[4]) {
-    const uint64_t g = e >> 3;
-    const uint4 w = philox4x32_10(make_uint4((uint32_t)g, (uint32_t)(g >> 32), (uint32_t)offset, (uint32_t)(offset >> 32)), keys);
-    const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
-    const uint64_t k2 = f2_pack(1.52587890625e-05f, 1.52587890625e-05f), c2 = f2_pack(-128.5f, -128.5f);
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-        out[j] = f2_fma(f2_pack(__uint_as_float(__byte_perm(ws[j], 0x4B000000u, 0x7410)), __uint_as_float(__byte_perm(ws[j], 0x4B000000u, 0x7432))), k2, c2);
+// The noise of the two elements of one generator word: both halves are placed over the exponent of 2^23 and rescaled by one two-wide FMA.
+__device__ __forceinline__ uint64_t noise2(uint32_t w) {
+    return f2_fma(f2_pack(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7410)), __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7432))),
+                  f2_pack(1.52587890625e-05f, 1.52587890625e-05f), f2_pack(-128.5f, -128.5f));
 }
+// Noise for the 8 consecutive elements starting at linear index e (e % 8 == 0), as four packed pairs.
+template <bool WIDE>
+__device__ __forceinline__ void philox_noise8x2(uint64_t e, const PhiloxKeys& keys, uint64_t offset, uint64_t (&out)[4]) {
+    const uint4 w = philox_group<WIDE>(e >> 3, keys, offset);
+    out[0] = noise2(w.x); out[1] = noise2(w.y); out[2] = noise2(w.z); out[3] = noise2(w.w);
+}
+// Where the noise of a launch comes from
+enum Noise : int { NOISE_GIVEN = 0, NOISE_PHILOX = 1, NOISE_PHILOX_WIDE = 2 };
+constexpr int64_t PHILOX_WIDE_ELEMENTS = int64_t(1) << 35;      // 8 elements per group number
+// v + sign(v) * noise for two values, i.e. sign(v) * (|v| + noise): rounding is symmetric, so the sign moves to the noise
+__device__ __forceinline__ uint64_t f2_add_noise(uint64_t v2, uint64_t nz2) { return f2_add(v2, nz2 ^ (v2 & 0x8000000080000000ull)); }
 
 // dtype-generic 16-element row chunk loads -> fp32
 template <typename T>

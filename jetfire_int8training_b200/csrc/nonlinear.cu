@@ -128,8 +128,11 @@ struct SrCfg {
     const float* noise;
     uint64_t offset;
     PhiloxKeys keys;
+    bool wide;          // the tensor has 2^35 elements or more
 };
-static inline SrCfg make_sr(const float* noise, uint64_t seed, uint64_t offset) { return SrCfg{noise, offset, make_philox_keys(seed)}; }
+static inline SrCfg make_sr(const float* noise, uint64_t seed, uint64_t offset, int64_t M, int64_t N) {
+    return SrCfg{noise, offset, make_philox_keys(seed, offset), M > 0 && N > 0 && M >= PHILOX_WIDE_ELEMENTS / N};
+}
 
 // low bytes of four registers -> one word
 __device__ __forceinline__ uint32_t gather_bytes(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
@@ -175,78 +178,99 @@ __device__ __forceinline__ void store_tile_transposed(const uint32_t* tile_words
     }
 }
 
+// One value of the explicit-noise / div.rn paths: quotient x, stochastic pre-step sign(x) * min(|x| + noise, 127) of the reference (its
+// lower clamp at -128 can never bind), rounding to the payload bits.
+template <bool TRUNC>
+__device__ __forceinline__ uint32_t round_bits(float x) { return TRUNC ? (uint32_t)__float2int_rz(x) : __float_as_uint(__fadd_rn(x, 12582912.0f)); }
+__device__ __forceinline__ float noisy(float x, float nz) {
+    return __uint_as_float(__float_as_uint(fminf(__fadd_rn(fabsf(x), nz), 127.f)) ^ (__float_as_uint(x) & 0x80000000u));
+}
+// The payload bits of two values given as a pair of dividends.  FAST: exact quotient by the Markstein sequence.  SR with generated noise
+// (PHILOX) needs no clamp on the fast path: scale32 = RN(absmax / 127), so |x| <= 127 + 2^-17, and the noise is at most 0.5 - 2^-16: the
+// sum stays below 127.5.
+template <bool FAST, bool TRUNC, bool SR, bool PHILOX>
+__device__ __forceinline__ void quantise2(uint64_t a2, uint64_t nz2, const Divisor& d, uint64_t inv2, uint64_t negb2, uint32_t& b0, uint32_t& b1) {
+    float x0, x1;
+    if (FAST && (PHILOX || !SR)) {
+        uint64_t x2 = f2_div_fast(a2, inv2, negb2);
+        if (SR) x2 = f2_add_noise(x2, nz2);
+        if (!TRUNC) x2 = f2_add(x2, f2_pack(12582912.0f, 12582912.0f));
+        f2_unpack(x2, x0, x1);
+        b0 = TRUNC ? (uint32_t)__float2int_rz(x0) : __float_as_uint(x0);
+        b1 = TRUNC ? (uint32_t)__float2int_rz(x1) : __float_as_uint(x1);
+        return;
+    }
+    if (FAST) {
+        f2_unpack(f2_div_fast(a2, inv2, negb2), x0, x1);
+    } else {
+        f2_unpack(a2, x0, x1);
+        x0 = __fdiv_rn(x0, d.b); x1 = __fdiv_rn(x1, d.b);
+    }
+    if (SR) {
+        float n0, n1;
+        f2_unpack(nz2, n0, n1);
+        x0 = noisy(x0, n0); x1 = noisy(x1, n1);
+    }
+    b0 = round_bits<TRUNC>(x0);
+    b1 = round_bits<TRUNC>(x1);
+}
+// One decision per warp each: the Markstein path is exact only inside its exponent window, and the noise is generated or given.  The
+// paths are separate instantiations of rows(fast, noise) (a run-time flag inside the element loop keeps all alive for every element).
+template <bool SR, class Rows>
+__device__ __forceinline__ void choose_path(Rows&& rows, bool fast, const SrCfg& sr) {
+    using T_ = std::true_type; using F_ = std::false_type;
+    using G_ = std::integral_constant<int, NOISE_GIVEN>; using P_ = std::integral_constant<int, NOISE_PHILOX>;
+    using W_ = std::integral_constant<int, NOISE_PHILOX_WIDE>;
+    if (!SR || (!sr.noise && !sr.wide && fast)) { if (fast) rows(T_{}, P_{}); else rows(F_{}, P_{}); }
+    else if (sr.noise)                          { if (fast) rows(T_{}, G_{}); else rows(F_{}, G_{}); }
+    else                                        { if (fast) rows(T_{}, W_{}); else rows(F_{}, W_{}); }      // wide, or div.rn
+}
+
 // Quantise the lane's NP x 16 values (row i delivered by rowf(i, a)) with the block scale `scale32` (= block absmax (+adj) / 127, identical in the lanes of a
-// block) and store payload + scale.  TRUNC selects the truncating conversion of the residual-add kernels; SR the stochastic
-// pre-step sign(v) * min(|v| + noise, 127) of the reference (its lower clamp at -128 can never bind).
-template <int TW, bool TRUNC, bool SR, bool TRANSPOSE, class RowF>
+// block) and store payload + scale.
+template <int TW, bool SR, bool TRANSPOSE, class RowF>
 __device__ __forceinline__ void emit_quantized(RowF&& rowf, float scale32, const Tile& t, int64_t M, int64_t N,
                                                int8_t* q, __half* s, const SrCfg& sr, uint32_t* tile_words, int8_t* qt) {
     constexpr int NP = Geo<TW>::NP;
     const Divisor d = make_divisor(scale32);
     const bool zero = (scale32 == 0.f);
-    // One decision per warp: the Markstein path is exact only inside its exponent window.  The two paths are separate
-    // instantiations of the loop (a run-time flag inside the element loop keeps both alive for every element).
     const bool fast = __all_sync(0xffffffffu, d.fast || zero);
-    const uint64_t inv2 = f2_pack(d.inv, d.inv), negb2 = f2_pack(-d.b, -d.b), magic2 = f2_pack(12582912.0f, 12582912.0f);
-    auto rows = [&](auto fast_c) {
-    constexpr bool FAST = decltype(fast_c)::value;
+    const uint64_t inv2 = f2_pack(d.inv, d.inv), negb2 = f2_pack(-d.b, -d.b);
+    choose_path<SR>([&](auto fast_c, auto noise_c) {
+        constexpr bool FAST = decltype(fast_c)::value, PHILOX = decltype(noise_c)::value != NOISE_GIVEN;
+        constexpr bool WIDE = decltype(noise_c)::value == NOISE_PHILOX_WIDE;
 #pragma unroll
-    for (int i = 0; i < NP; ++i) {
-        const int64_t row = row_of<TW>(t, i);
-        uint32_t words[4] = {0u, 0u, 0u, 0u};
-        if (t.active) {
-            float av[16];
-            rowf(i, av);
-            float nz[16];
-            if (SR) {
-                if (sr.noise) {
-                    const float4* np4 = reinterpret_cast<const float4*>(sr.noise + row * N + t.col);
+        for (int i = 0; i < NP; ++i) {
+            const int64_t row = row_of<TW>(t, i);
+            uint32_t words[4] = {0u, 0u, 0u, 0u};
+            if (t.active) {
+                float av[16];
+                rowf(i, av);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const float4 n4 = __ldg(np4 + k);
-                        nz[4 * k] = n4.x; nz[4 * k + 1] = n4.y; nz[4 * k + 2] = n4.z; nz[4 * k + 3] = n4.w;
+                for (int h = 0; h < 2; ++h) {            // 8 elements = one Philox call
+                    uint64_t nz2[4] = {0ull, 0ull, 0ull, 0ull};
+                    if (SR && PHILOX) {
+                        philox_noise8x2<WIDE>((uint64_t)(row * N + t.col) + 8 * h, sr.keys, sr.offset, nz2);
+                    } else if (SR) {
+                        const float4* np4 = reinterpret_cast<const float4*>(sr.noise + row * N + t.col + 8 * h);
+                        const float4 n0 = __ldg(np4), n1 = __ldg(np4 + 1);
+                        nz2[0] = f2_pack(n0.x, n0.y); nz2[1] = f2_pack(n0.z, n0.w); nz2[2] = f2_pack(n1.x, n1.y); nz2[3] = f2_pack(n1.z, n1.w);
                     }
-                } else {
-                    philox_noise8((uint64_t)(row * N + t.col), sr.keys, sr.offset, &nz[0]);
-                    philox_noise8((uint64_t)(row * N + t.col) + 8, sr.keys, sr.offset, &nz[8]);
+                    uint32_t b[8];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        quantise2<FAST, false, SR, PHILOX>(f2_pack(av[8 * h + 2 * u], av[8 * h + 2 * u + 1]), nz2[u], d, inv2, negb2, b[2 * u], b[2 * u + 1]);
+                    words[2 * h] = zero ? 0u : gather_bytes(b[0], b[1], b[2], b[3]);
+                    words[2 * h + 1] = zero ? 0u : gather_bytes(b[4], b[5], b[6], b[7]);
                 }
+                *reinterpret_cast<int4*>(q + row * N + t.col) = make_int4(words[0], words[1], words[2], words[3]);
             }
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                uint32_t b[4];
-#pragma unroll
-                for (int j = 0; j < 4; j += 2) {
-                    float x0, x1;
-                    if (FAST) {
-                        const uint64_t x2 = f2_div_fast(f2_pack(av[4 * k + j], av[4 * k + j + 1]), inv2, negb2);
-                        if (!SR && !TRUNC) {
-                            f2_unpack(f2_add(x2, magic2), x0, x1);
-                            b[j] = __float_as_uint(x0); b[j + 1] = __float_as_uint(x1);
-                            continue;
-                        }
-                        f2_unpack(x2, x0, x1);
-                    } else {
-                        x0 = __fdiv_rn(av[4 * k + j], d.b); x1 = __fdiv_rn(av[4 * k + j + 1], d.b);
-                    }
-                    if (SR) {
-                        const float m0 = fminf(__fadd_rn(fabsf(x0), nz[4 * k + j]), 127.f), m1 = fminf(__fadd_rn(fabsf(x1), nz[4 * k + j + 1]), 127.f);
-                        x0 = __uint_as_float(__float_as_uint(m0) ^ (__float_as_uint(x0) & 0x80000000u));
-                        x1 = __uint_as_float(__float_as_uint(m1) ^ (__float_as_uint(x1) & 0x80000000u));
-                    }
-                    b[j] = TRUNC ? (uint32_t)__float2int_rz(x0) : __float_as_uint(__fadd_rn(x0, 12582912.0f));
-                    b[j + 1] = TRUNC ? (uint32_t)__float2int_rz(x1) : __float_as_uint(__fadd_rn(x1, 12582912.0f));
-                }
-                words[k] = zero ? 0u : gather_bytes(b[0], b[1], b[2], b[3]);
+            if (TRANSPOSE) {
+                uint32_t* dst = tile_words + (i * Geo<TW>::RPP + t.rg) * (TW / 4) + t.cc * 4;
+                *reinterpret_cast<int4*>(dst) = make_int4(words[0], words[1], words[2], words[3]);
             }
-            *reinterpret_cast<int4*>(q + row * N + t.col) = make_int4(words[0], words[1], words[2], words[3]);
         }
-        if (TRANSPOSE) {
-            uint32_t* dst = tile_words + (i * Geo<TW>::RPP + t.rg) * (TW / 4) + t.cc * 4;
-            *reinterpret_cast<int4*>(dst) = make_int4(words[0], words[1], words[2], words[3]);
-        }
-    }
-    };
-    if (fast) rows(std::true_type{}); else rows(std::false_type{});
+    }, fast, sr);
     if (t.active && t.rg == 0 && (t.cc & 1) == 0) s[t.tm * (N / QB) + (t.col >> 5)] = __float2half_rn(scale32);
     if (TRANSPOSE) {
         __syncwarp();
@@ -368,6 +392,29 @@ __device__ __forceinline__ void widen16(const uint4 (&d)[2], float (&v)[16], __n
     }
 }
 
+// max |x| of the 16 values of a row chunk: 16-bit inputs two at a time (NaN is ignored, as by fmaxf)
+__device__ __forceinline__ float absmax16(const uint4 (&d)[4], float) {
+    float m = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        m = fmaxf(m, fmaxf(fmaxf(fabsf(__uint_as_float(d[k].x)), fabsf(__uint_as_float(d[k].y))),
+                           fmaxf(fabsf(__uint_as_float(d[k].z)), fabsf(__uint_as_float(d[k].w)))));
+    return m;
+}
+template <typename T2>
+__device__ __forceinline__ T2 absmax_words(const uint4& v) {
+    const T2* h = reinterpret_cast<const T2*>(&v);
+    return __hmax2(__hmax2(__habs2(h[0]), __habs2(h[1])), __hmax2(__habs2(h[2]), __habs2(h[3])));
+}
+__device__ __forceinline__ float absmax16(const uint4 (&d)[2], __half) {
+    const float2 f = __half22float2(__hmax2(absmax_words<__half2>(d[0]), absmax_words<__half2>(d[1])));
+    return fmaxf(fmaxf(f.x, f.y), 0.f);
+}
+__device__ __forceinline__ float absmax16(const uint4 (&d)[2], __nv_bfloat16) {
+    const float2 f = __bfloat1622float2(__hmax2(absmax_words<__nv_bfloat162>(d[0]), absmax_words<__nv_bfloat162>(d[1])));
+    return fmaxf(fmaxf(f.x, f.y), 0.f);
+}
+
 // =========================================================================================================
 // quantize / quantize_transpose.  The tile stays packed in registers; it is widened once for the block absmax and once more
 // for the quantisation, which is cheaper than holding 64 fp32 values next to the prefetched next tile.
@@ -386,14 +433,9 @@ quantize_kernel(const T* __restrict__ x, int64_t M, int64_t N, int8_t* __restric
         [&](const Tile& t, Raw& r) {
             float m = 0.f;
 #pragma unroll
-            for (int i = 0; i < NP; ++i) {
-                float a[16];
-                widen16(r.d[i], a, T());
-#pragma unroll
-                for (int j = 0; j < 16; ++j) m = fmaxf(m, fabsf(a[j]));
-            }
+            for (int i = 0; i < NP; ++i) m = fmaxf(m, absmax16(r.d[i], T()));
             const float scale32 = __fdiv_rn(block_max<TW>(m), 127.0f);
-            emit_quantized<TW, false, SR, TRANSPOSE>([&](int i, float (&a)[16]) { widen16(r.d[i], a, T()); }, scale32, t, M, N, q, s, sr,
+            emit_quantized<TW, SR, TRANSPOSE>([&](int i, float (&a)[16]) { widen16(r.d[i], a, T()); }, scale32, t, M, N, q, s, sr,
                                                      tile_words, qt);
         });
 }
@@ -714,7 +756,7 @@ gelu_bwd_kernel(const int8_t* __restrict__ qx, const __half* __restrict__ sx, co
                     f2_unpack(f2_mul(f2_pack(fd[j], fd[j + 1]), f2_mul(f2_pack(fg[j], fg[j + 1]), scg2)), v[i][j], v[i][j + 1]);
             }
             const float scale32 = __fdiv_rn(block_max<TW>(absmax_tile<NP>(v)), 127.0f);
-            emit_quantized<TW, false, SR, false>([&](int i, float (&a)[16]) {
+            emit_quantized<TW, SR, false>([&](int i, float (&a)[16]) {
 #pragma unroll
                 for (int j = 0; j < 16; ++j) a[j] = v[i][j];
             }, scale32, t, M, N, qd, sd, sr, nullptr, nullptr);
@@ -763,7 +805,7 @@ ln_fwd_kernel(const int8_t* __restrict__ qx, const __half* __restrict__ sx, cons
             }
             const float scale32 = __fdiv_rn(block_max<TW>(absmax_tile<NP>(v)), 127.0f);
             SrCfg sr{};
-            emit_quantized<TW, false, false, false>([&](int i, float (&a)[16]) {
+            emit_quantized<TW, false, false>([&](int i, float (&a)[16]) {
 #pragma unroll
                 for (int j = 0; j < 16; ++j) a[j] = v[i][j];
             }, scale32, t, M, N, qy, sy, sr, nullptr, nullptr);
@@ -872,7 +914,7 @@ ln_bwd_kernel(const int8_t* __restrict__ qx, const __half* __restrict__ sx, cons
     }
     const float amax = block_max<TW>(absmax_tile<NP>(v));   // exactly representable in fp16
     const float scale32 = __fdiv_rn(amax, 127.0f);
-    emit_quantized<TW, false, SR, false>([&](int i, float (&a)[16]) {
+    emit_quantized<TW, SR, false>([&](int i, float (&a)[16]) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) a[j] = v[i][j];
     }, scale32, t, M, N, qd, sd, sr, nullptr, nullptr);
@@ -918,71 +960,42 @@ __device__ __forceinline__ void emit_block4(RowF&& rowf /* i -> the lane's float
     const Divisor d = make_divisor(scale32);
     const bool zero = (scale32 == 0.f);
     const bool fast = d.fast || zero;                      // identical in every lane: one divisor per block
-    const uint64_t inv2 = f2_pack(d.inv, d.inv), negb2 = f2_pack(-d.b, -d.b), magic2 = f2_pack(12582912.0f, 12582912.0f);
-    auto rows = [&](auto fast_c) {
-        constexpr bool FAST = decltype(fast_c)::value;
+    const uint64_t inv2 = f2_pack(d.inv, d.inv), negb2 = f2_pack(-d.b, -d.b);
+    choose_path<SR>([&](auto fast_c, auto noise_c) {
+        constexpr bool FAST = decltype(fast_c)::value, PHILOX = decltype(noise_c)::value != NOISE_GIVEN;
+        constexpr bool WIDE = decltype(noise_c)::value == NOISE_PHILOX_WIDE;
 #pragma unroll
         for (int i2 = 0; i2 < 8; i2 += 2) {
-            float nz[2][4];
-            if (SR) {
-                if (sr.noise) {
+            uint64_t nz2[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
+            if (SR && !PHILOX) {
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const float4 n4 = __ldg(reinterpret_cast<const float4*>(sr.noise + base + (int64_t)(4 * (i2 + h)) * N));
-                        nz[h][0] = n4.x; nz[h][1] = n4.y; nz[h][2] = n4.z; nz[h][3] = n4.w;
-                    }
-                } else {
-                    // this lane generates the 8-element group of pass i2 (even c) or i2 + 1 (odd c); a group starts at the even
-                    // lane's first column
-                    const int odd = c & 1;
-                    const uint64_t e = (uint64_t)(base + (int64_t)(4 * (i2 + odd)) * N - 4 * odd);
-                    float g8[8];
-                    philox_noise8(e, sr.keys, sr.offset, g8);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        // keep the half over this lane's own columns; the other half is the neighbour's (even lane: high half of
-                        // pass i2's group, odd lane: low half of pass i2+1's group)
-                        const float got = __shfl_xor_sync(0xffffffffu, odd ? g8[k] : g8[4 + k], 1);
-                        const float own = odd ? g8[4 + k] : g8[k];
-                        nz[0][k] = odd ? got : own;       // (selects, not a run-time array index: that would put nz in local memory)
-                        nz[1][k] = odd ? own : got;
-                    }
+                for (int h = 0; h < 2; ++h) {
+                    const float4 n4 = __ldg(reinterpret_cast<const float4*>(sr.noise + base + (int64_t)(4 * (i2 + h)) * N));
+                    nz2[h][0] = f2_pack(n4.x, n4.y); nz2[h][1] = f2_pack(n4.z, n4.w);
                 }
+            } else if (SR) {
+                // this lane generates the 8-element group of pass i2 (even c) or i2 + 1 (odd c); a group starts at the even
+                // lane's first column.  It keeps the half over its own columns (even lane: low half of pass i2's group, odd lane: high
+                // half of pass i2 + 1's) and sends the other one -- two raw words, not four noise values -- to its neighbour.
+                const int odd = c & 1;
+                const uint64_t e = (uint64_t)(base + (int64_t)(4 * (i2 + odd)) * N - 4 * odd);
+                const uint4 w = philox_group<WIDE>(e >> 3, sr.keys, sr.offset);
+                const uint32_t got0 = __shfl_xor_sync(0xffffffffu, odd ? w.x : w.z, 1), got1 = __shfl_xor_sync(0xffffffffu, odd ? w.y : w.w, 1);
+                const uint32_t own0 = odd ? w.z : w.x, own1 = odd ? w.w : w.y;
+                nz2[0][0] = noise2(odd ? got0 : own0); nz2[0][1] = noise2(odd ? got1 : own1);
+                nz2[1][0] = noise2(odd ? own0 : got0); nz2[1][1] = noise2(odd ? own1 : got1);
             }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int i = i2 + h;
-                const float4 vi = rowf(i);
-                const float a[4] = {vi.x, vi.y, vi.z, vi.w};
-                uint32_t bts[4];
-#pragma unroll
-                for (int k = 0; k < 4; k += 2) {
-                    float x0, x1;
-                    if (FAST) {
-                        const uint64_t x2 = f2_div_fast(f2_pack(a[k], a[k + 1]), inv2, negb2);
-                        if (!SR && !TRUNC) {
-                            f2_unpack(f2_add(x2, magic2), x0, x1);
-                            bts[k] = __float_as_uint(x0); bts[k + 1] = __float_as_uint(x1);
-                            continue;
-                        }
-                        f2_unpack(x2, x0, x1);
-                    } else {
-                        x0 = __fdiv_rn(a[k], d.b); x1 = __fdiv_rn(a[k + 1], d.b);
-                    }
-                    if (SR) {
-                        const float m0 = fminf(__fadd_rn(fabsf(x0), nz[h][k]), 127.f), m1 = fminf(__fadd_rn(fabsf(x1), nz[h][k + 1]), 127.f);
-                        x0 = __uint_as_float(__float_as_uint(m0) ^ (__float_as_uint(x0) & 0x80000000u));
-                        x1 = __uint_as_float(__float_as_uint(m1) ^ (__float_as_uint(x1) & 0x80000000u));
-                    }
-                    bts[k] = TRUNC ? (uint32_t)__float2int_rz(x0) : __float_as_uint(__fadd_rn(x0, 12582912.0f));
-                    bts[k + 1] = TRUNC ? (uint32_t)__float2int_rz(x1) : __float_as_uint(__fadd_rn(x1, 12582912.0f));
-                }
-                const uint32_t word = zero ? 0u : gather_bytes(bts[0], bts[1], bts[2], bts[3]);
-                *reinterpret_cast<uint32_t*>(qy + base + (int64_t)(4 * i) * N) = word;
+                const float4 v = rowf(i);
+                uint32_t b[4];
+                quantise2<FAST, TRUNC, SR, PHILOX>(f2_pack(v.x, v.y), nz2[h][0], d, inv2, negb2, b[0], b[1]);
+                quantise2<FAST, TRUNC, SR, PHILOX>(f2_pack(v.z, v.w), nz2[h][1], d, inv2, negb2, b[2], b[3]);
+                *reinterpret_cast<uint32_t*>(qy + base + (int64_t)(4 * i) * N) = zero ? 0u : gather_bytes(b[0], b[1], b[2], b[3]);
             }
         }
-    };
-    if (fast) rows(std::true_type{}); else rows(std::false_type{});
+    }, fast, sr);
 }
 
 // quantize without the transposed copy, in the same mapping: a warp owns one 32x32 block, persistent over the blocks with the
@@ -1319,7 +1332,7 @@ int jf_int8_quantize(const void* x, int x_dtype, int64_t M, int64_t N, int8_t* q
     if (qt) JF_REQUIRE_ALIGNED(qt);
     if (noise) JF_REQUIRE_ALIGNED(noise);
     cudaStream_t st = (cudaStream_t)stream;
-    SrCfg sr = make_sr(noise, seed, offset);
+    SrCfg sr = make_sr(noise, seed, offset, M, N);
     __half* sh = (__half*)s;
     const bool sto = stochastic != 0;
     switch (x_dtype) {
@@ -1399,7 +1412,7 @@ int jf_int8_gelu_backward(const int8_t* qx, const void* sx, const int8_t* qg, co
     if (int e = check_mn(M, N)) return e;
     JF_REQUIRE_ALIGNED(qx); JF_REQUIRE_ALIGNED(qg); JF_REQUIRE_ALIGNED(qd);
     if (noise) JF_REQUIRE_ALIGNED(noise);
-    SrCfg sr = make_sr(noise, seed, offset);
+    SrCfg sr = make_sr(noise, seed, offset, M, N);
     cudaStream_t st = (cudaStream_t)stream;
     const __half* sxh = (const __half*)sx; const __half* sgh = (const __half*)sg; __half* sdh = (__half*)sd;
     if (int e = ensure_gelu_table(st, true)) return e;
@@ -1432,7 +1445,7 @@ int jf_int8_layernorm_backward(const int8_t* qx, const void* sx, const int8_t* q
     JF_REQUIRE_ALIGNED(qx); JF_REQUIRE_ALIGNED(qg); JF_REQUIRE_ALIGNED(qd); JF_REQUIRE_ALIGNED(gamma); JF_REQUIRE_ALIGNED(scratch);
     if (noise) JF_REQUIRE_ALIGNED(noise);
     cudaStream_t st = (cudaStream_t)stream;
-    SrCfg sr = make_sr(noise, seed, offset);
+    SrCfg sr = make_sr(noise, seed, offset, M, N);
     const int64_t slab_tiles = (M / QB) * ((N + 127) / 128);
     const unsigned grid = (unsigned)((slab_tiles + WARPS / 2 - 1) / (WARPS / 2));   // two warps per 32 x 128 slab tile
     const __half* sxh = (const __half*)sx; const __half* sgh = (const __half*)sg; __half* sdh = (__half*)sd;
@@ -1475,7 +1488,7 @@ static int add_impl(const void* x1, int x1_dtype, const int8_t* q2, const void* 
 
 int jf_int8_add(const void* x1, int x1_dtype, const int8_t* q2, const void* s2, int64_t M, int64_t N, float* y1, int8_t* qy, void* sy,
                 int stochastic, const float* noise, uint64_t seed, uint64_t offset, void* stream) {
-    SrCfg sr = make_sr(noise, seed, offset);
+    SrCfg sr = make_sr(noise, seed, offset, M, N);
     return add_impl(x1, x1_dtype, q2, s2, M, N, y1, qy, sy, nullptr, nullptr, nullptr, false, stochastic != 0, sr, (cudaStream_t)stream);
 }
 
