@@ -84,6 +84,7 @@ __device__ __forceinline__ bool lean_wait(uint64_t* bar, uint32_t parity, volati
 template <bool A_MN, bool B_MN, int CONV>
 __global__ void __launch_bounds__(GEMM_THREADS, 2)
 gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
+    grid_launch_dependents();      // the split-K reduction, where there is one
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     // barriers: pair_full[2] at 0, pair_empty[2] at 16, abort flag at 32, tmem slot at 36, drain at 40, full[STAGES] at 48,

@@ -24,6 +24,29 @@ inline int check_launch() {
     }
     return JF_OK;
 }
+// The second kernel of a reduction: it is launched while the first one, which has said grid_launch_dependents(), still runs, and waits for
+// its results with grid_dependency_wait(), so that its own launch costs no gap (~1 us of a 10 us call).  (Its input pointers carry no
+// __restrict__: a load through the non-coherent path may not start before the wait.)
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class... P, class... A>
+inline int launch_dependent(void (*kernel)(P...), unsigned grid, unsigned threads, cudaStream_t st, A... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    if (e != cudaSuccess) {
+        g_last_cuda_error = (int)e;
+        return JF_ERR_LAUNCH;
+    }
+    return JF_OK;
+}
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 inline bool mult32(int64_t v) { return v > 0 && (v % 32) == 0; }
 

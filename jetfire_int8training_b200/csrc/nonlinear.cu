@@ -827,6 +827,7 @@ ln_bwd_kernel(const int8_t* __restrict__ qx, const __half* __restrict__ sx, cons
               const float* __restrict__ rstd, int64_t M, int64_t N, int8_t* __restrict__ qd, __half* __restrict__ sd,
               float* __restrict__ dw_partial, SrCfg sr) {
     constexpr int NP = Geo<TW>::NP, WPS = 128 / TW, PAIRS = WARPS / WPS;   // WPS warps per slab tile, PAIRS slab tiles per CTA
+    grid_launch_dependents();                          // the dgamma reduction
     __shared__ float2 row_part[PAIRS][WPS][QB];        // [slab tile][part][row of the tile] = (sum xhat*wdy, sum wdy) over the part
     const int warp = threadIdx.x >> 5, pair = warp / WPS, half = warp % WPS;
     const int64_t slabs_n = (N + 127) / 128, tiles_n_ = (N + TW - 1) / TW;
@@ -849,10 +850,13 @@ ln_bwd_kernel(const int8_t* __restrict__ qx, const __half* __restrict__ sx, cons
         for (int j = 0; j < 16; ++j) gm[j] = 0.f;
     }
     const float n_f = (float)N;
-    float v[NP][16];    // dx, rounded to fp16 and widened
-    float dwp[16];      // partial dgamma over this lane's rows
+    uint64_t gm2[8];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) dwp[j] = 0.f;
+    for (int j = 0; j < 8; ++j) gm2[j] = f2_pack(gm[2 * j], gm[2 * j + 1]);
+    __half2 v16[NP][8];    // dx, rounded to fp16 (kept packed: half the registers, and the block absmax takes two values per instruction)
+    uint64_t dwp2[8];      // partial dgamma over this lane's rows
+#pragma unroll
+    for (int j = 0; j < 8; ++j) dwp2[j] = 0ull;
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
         const int64_t row = row_of<TW>(t, i);
@@ -861,7 +865,7 @@ ln_bwd_kernel(const int8_t* __restrict__ qx, const __half* __restrict__ sx, cons
         const __half rs16 = __float2half_rn(__ldg(rstd + row));
         const __half2 rs2 = __half2half2(rs16);
         const float rs = __half2float(rs16);
-        float xh[16], wdy[16];
+        uint64_t xh2[8], wdy2[8];
         __half2 hx[8], hg[8];
         unpack16_h2(rx[i], hx);
         unpack16_h2(rgr[i], hg);
@@ -872,11 +876,14 @@ ln_bwd_kernel(const int8_t* __restrict__ qx, const __half* __restrict__ sx, cons
             const __half2 dy16 = __hmul2_rn(hg[j], sg2);
             const __half2 xhat16 = __hmul2_rn(__hsub2_rn(x16, mu2), rs2);
             const float2 xf = __half22float2(xhat16), dyf = __half22float2(dy16), pr = __half22float2(__hmul2_rn(dy16, xhat16));
-            xh[2 * j] = xf.x; xh[2 * j + 1] = xf.y;
-            wdy[2 * j] = __fmul_rn(gm[2 * j], dyf.x); wdy[2 * j + 1] = __fmul_rn(gm[2 * j + 1], dyf.y);
-            s1 = __fadd_rn(__fadd_rn(s1, __fmul_rn(xh[2 * j], wdy[2 * j])), __fmul_rn(xh[2 * j + 1], wdy[2 * j + 1]));
-            s2 = __fadd_rn(__fadd_rn(s2, wdy[2 * j]), wdy[2 * j + 1]);
-            dwp[2 * j] = __fadd_rn(dwp[2 * j], pr.x); dwp[2 * j + 1] = __fadd_rn(dwp[2 * j + 1], pr.y);
+            xh2[j] = f2_pack(xf.x, xf.y);
+            wdy2[j] = f2_mul(gm2[j], f2_pack(dyf.x, dyf.y));
+            float p0, p1, w0, w1;
+            f2_unpack(f2_mul(xh2[j], wdy2[j]), p0, p1);
+            f2_unpack(wdy2[j], w0, w1);
+            s1 = __fadd_rn(__fadd_rn(s1, p0), p1);
+            s2 = __fadd_rn(__fadd_rn(s2, w0), w1);
+            dwp2[j] = f2_add(dwp2[j], f2_pack(pr.x, pr.y));
         }
         // sums over this warp's 64 columns, then the other warp's through shared memory (left + right)
         s1 = row_sum<TW>(s1);
@@ -897,14 +904,16 @@ ln_bwd_kernel(const int8_t* __restrict__ qx, const __half* __restrict__ sx, cons
 #pragma unroll
         for (int j = 0; j < 16; j += 2) {
             // (wdy - (xhat * c1 + c2)) * rstd, each operation rounded:  -(a*b + c) == (a * -b) + -c  exactly
-            const uint64_t ntt = f2_add(f2_mul(f2_pack(xh[j], xh[j + 1]), nc1), nc2);
+            const uint64_t ntt = f2_add(f2_mul(xh2[j / 2], nc1), nc2);
             float d0, d1;
-            f2_unpack(f2_mul(f2_add(f2_pack(wdy[j], wdy[j + 1]), ntt), rs_2), d0, d1);
-            const float2 dd = __half22float2(__floats2half2_rn(d0, d1));
-            v[i][j] = dd.x; v[i][j + 1] = dd.y;
+            f2_unpack(f2_mul(f2_add(wdy2[j / 2], ntt), rs_2), d0, d1);
+            v16[i][j / 2] = __floats2half2_rn(d0, d1);
         }
     }
     // partial dgamma: reduce the row groups, lanes with rg == 0 write 16 columns
+    float dwp[16];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f2_unpack(dwp2[j], dwp[2 * j], dwp[2 * j + 1]);
 #pragma unroll
     for (int j = 0; j < 16; ++j) dwp[j] = col_sum<TW>(dwp[j]);
     if (t.active && t.rg == 0) {
@@ -912,23 +921,41 @@ ln_bwd_kernel(const int8_t* __restrict__ qx, const __half* __restrict__ sx, cons
 #pragma unroll
         for (int k = 0; k < 4; ++k) dst[k] = make_float4(dwp[4 * k], dwp[4 * k + 1], dwp[4 * k + 2], dwp[4 * k + 3]);
     }
-    const float amax = block_max<TW>(absmax_tile<NP>(v));   // exactly representable in fp16
-    const float scale32 = __fdiv_rn(amax, 127.0f);
+    __half2 m2 = __floats2half2_rn(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < NP; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) m2 = __hmax2(m2, __habs2(v16[i][j]));
+    const float2 mf = __half22float2(m2);
+    const float scale32 = __fdiv_rn(block_max<TW>(fmaxf(mf.x, mf.y)), 127.0f);
     emit_quantized<TW, SR, false>([&](int i, float (&a)[16]) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) a[j] = v[i][j];
+        for (int j = 0; j < 8; ++j) {
+            const float2 f = __half22float2(v16[i][j]);
+            a[2 * j] = f.x; a[2 * j + 1] = f.y;
+        }
     }, scale32, t, M, N, qd, sd, sr, nullptr, nullptr);
 }
 
 // dgamma[n] = sum over the M/32 partial rows: 8 interleaved row groups per column (thread (x, g) sums rows g, g+8, ...), then the
 // 8 group sums in ascending order -- a fixed order, so the result is deterministic.  Block = 32 columns x 8 groups.
-__global__ void __launch_bounds__(256) ln_bwd_dw_kernel(const float* __restrict__ partial, int64_t rows, int64_t N, float* __restrict__ dgamma) {
+__global__ void __launch_bounds__(256) ln_bwd_dw_kernel(const float* partial, int64_t rows, int64_t N, float* __restrict__ dgamma) {
     __shared__ float red[8][32];
     const int tx = threadIdx.x & 31, g = threadIdx.x >> 5;
     const int64_t n = (int64_t)blockIdx.x * 32 + tx;
+    grid_dependency_wait();
     float a = 0.f;
-    if (n < N)
-        for (int64_t r = g; r < rows; r += 8) a = __fadd_rn(a, partial[r * N + n]);
+    if (n < N) {
+        int64_t r = g;
+        for (; r + 7 * 8 < rows; r += 8 * 8) {            // eight loads in flight, summed in order
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = partial[(r + 8 * k) * N + n];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) a = __fadd_rn(a, v[k]);
+        }
+        for (; r < rows; r += 8) a = __fadd_rn(a, partial[r * N + n]);
+    }
     red[g][tx] = a;
     __syncthreads();
     if (g == 0 && n < N) {
@@ -1452,8 +1479,7 @@ int jf_int8_layernorm_backward(const int8_t* qx, const void* sx, const int8_t* q
     if (stochastic) ln_bwd_kernel<true><<<grid, THREADS, 0, st>>>(qx, sxh, qg, sgh, gamma, mean, rstd, M, N, qd, sdh, scratch, sr);
     else ln_bwd_kernel<false><<<grid, THREADS, 0, st>>>(qx, sxh, qg, sgh, gamma, mean, rstd, M, N, qd, sdh, scratch, sr);
     if (int e = check_launch()) return e;
-    ln_bwd_dw_kernel<<<(unsigned)((N + 31) / 32), 256, 0, st>>>(scratch, M / QB, N, dgamma);
-    return check_launch();
+    return launch_dependent(ln_bwd_dw_kernel, (unsigned)((N + 31) / 32), 256, st, (const float*)scratch, M / QB, N, dgamma);
 }
 
 static int add_impl(const void* x1, int x1_dtype, const int8_t* q2, const void* s2, int64_t M, int64_t N, float* y1, int8_t* qy,
