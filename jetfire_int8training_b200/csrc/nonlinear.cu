@@ -1132,7 +1132,8 @@ __global__ void __launch_bounds__(THREADS, 3) quantize_multi_kernel(const Quanti
 // The block absmax is a thread-local max + one redux.sync.  Stochastic rounding: one Philox call yields the noise of 8
 // consecutive elements = two neighbouring lanes; the even lane generates the call of the even passes, the odd lane that of the
 // odd passes, and they exchange the halves they owe each other with two shuffles per pair of passes.
-// With MEANVAR a warp walks the four blocks of a 128-column slab and writes one partial sum / sum of squares per row and slab.
+// With MEANVAR one partial sum / sum of squares per row and 128-column slab goes to scratch.  (One warp walking the four blocks of a slab
+// left [3104 x 1600] at 8 warps per SM; with a warp per block the operator takes 10.2 us instead of 14.4, 4.0 TB/s.)
 template <typename T>
 __device__ __forceinline__ float4 load4(const T* p);
 template <>
@@ -1150,25 +1151,38 @@ __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bfloat16* p) {
                        __uint_as_float(v.y & 0xFFFF0000u));
 }
 
+// Sum of eight per-lane values over the eight lanes of a row group: lane c ends with the total of value c.  Seven shuffles (the halves of
+// the value list are exchanged, then quarters, then eighths) instead of three per value.
+__device__ __forceinline__ float rowgroup_sum8(float (&v)[8], int c) {
+#pragma unroll
+    for (int mask = 4; mask >= 1; mask >>= 1)
+#pragma unroll
+        for (int k = 0; k < mask; ++k) {
+            const bool up = c & mask;                     // keep the upper half of the list
+            const float send = up ? v[k] : v[k + mask], keep = up ? v[k + mask] : v[k];
+            v[k] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, mask));
+        }
+    return v[0];
+}
+
 template <typename T, bool MEANVAR, bool SR>
 __global__ void __launch_bounds__(THREADS, 3)
 add_kernel(const T* __restrict__ x1, const int8_t* __restrict__ q2, const __half* __restrict__ s2, int64_t M, int64_t N,
            float* __restrict__ y1, int8_t* __restrict__ qy, __half* __restrict__ sy, float* __restrict__ part_sum,
            float* __restrict__ part_sq, SrCfg sr) {
-    constexpr int SUBS = MEANVAR ? 4 : 1;                     // 32-column blocks per work item
+    // Row statistics: the four warps of a 128-column slab leave their blocks' row sums in shared memory and are summed in column order.
+    __shared__ float2 row_part[MEANVAR ? WARPS : 1][MEANVAR ? QB : 1];
+    if (MEANVAR) grid_launch_dependents();                    // the statistics' last step
     const int64_t blocks_n = N / QB;                          // blocks per row of blocks
-    const int64_t groups_n = (blocks_n + SUBS - 1) / SUBS;    // work items per row of blocks (MEANVAR: 128-column slabs)
+    const int64_t slabs_n = (blocks_n + 3) / 4;               // MEANVAR: warps are numbered by slab, a short last slab leaves some idle
     const int64_t item = (int64_t)blockIdx.x * WARPS + (threadIdx.x >> 5);
-    if (item >= (M / QB) * groups_n) return;
-    const int64_t tm = (int64_t)((uint32_t)item / (uint32_t)groups_n), grp = (int64_t)((uint32_t)item % (uint32_t)groups_n);   // 32-bit division
-    const int lane = threadIdx.x & 31, r = lane >> 3, c = lane & 7;
-    float ps[8], pq[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) ps[i] = pq[i] = 0.f;
-#pragma unroll 1
-    for (int sub = 0; sub < SUBS; ++sub) {
-        const int64_t tn = grp * SUBS + sub;
-        if (tn >= blocks_n) break;                            // warp-uniform
+    const int64_t per_row = MEANVAR ? 4 * slabs_n : blocks_n;
+    const bool inside = item < (M / QB) * per_row;
+    const int64_t tm = (int64_t)((uint32_t)item / (uint32_t)per_row), tn = (int64_t)((uint32_t)item % (uint32_t)per_row);   // 32-bit division
+    const int lane = threadIdx.x & 31, r = lane >> 3, c = lane & 7, warp = threadIdx.x >> 5;
+    const bool live = inside && tn < blocks_n;                // warp-uniform
+    if (!MEANVAR && !live) return;
+    if (live) {
         const int64_t base = (tm * QB + r) * N + tn * QB + 4 * c;      // element (row r of the block, this lane's columns)
         uint32_t qw[8];
         float4 v[8];
@@ -1178,6 +1192,7 @@ add_kernel(const T* __restrict__ x1, const int8_t* __restrict__ q2, const __half
         for (int i = 0; i < 8; ++i) v[i] = load4<T>(x1 + base + (int64_t)(4 * i) * N);
         const float sc = __half2float(__ldg(s2 + tm * blocks_n + tn));
         float m = 0.f;
+        float ps[8], pq[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             v[i].x = __fadd_rn(v[i].x, __fmul_rn(byte_to_float(qw[i], 0), sc));
@@ -1187,38 +1202,42 @@ add_kernel(const T* __restrict__ x1, const int8_t* __restrict__ q2, const __half
             *reinterpret_cast<float4*>(y1 + base + (int64_t)(4 * i) * N) = v[i];
             m = fmaxf(fmaxf(m, fmaxf(fabsf(v[i].x), fabsf(v[i].y))), fmaxf(fabsf(v[i].z), fabsf(v[i].w)));
             if (MEANVAR) {
-                ps[i] = __fadd_rn(ps[i], __fadd_rn(__fadd_rn(v[i].x, v[i].y), __fadd_rn(v[i].z, v[i].w)));
-                pq[i] = __fadd_rn(pq[i], __fadd_rn(__fadd_rn(__fmul_rn(v[i].x, v[i].x), __fmul_rn(v[i].y, v[i].y)),
-                                                   __fadd_rn(__fmul_rn(v[i].z, v[i].z), __fmul_rn(v[i].w, v[i].w))));
+                ps[i] = __fadd_rn(__fadd_rn(v[i].x, v[i].y), __fadd_rn(v[i].z, v[i].w));
+                pq[i] = __fadd_rn(__fadd_rn(__fmul_rn(v[i].x, v[i].x), __fmul_rn(v[i].y, v[i].y)),
+                                  __fadd_rn(__fmul_rn(v[i].z, v[i].z), __fmul_rn(v[i].w, v[i].w)));
             }
         }
         const float amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
         const float scale32 = __fdiv_rn(amax, 127.0f);
+        if (MEANVAR) row_part[warp][4 * c + r] = make_float2(rowgroup_sum8(ps, c), rowgroup_sum8(pq, c));   // row 4 i + r, i = c
         emit_block4<true, SR>([&](int i) { return v[i]; }, scale32, base, N, c, qy, sr);
         if (lane == 0) sy[tm * blocks_n + tn] = __float2half_rn(scale32);
+    } else if (MEANVAR) {
+        row_part[warp][lane] = make_float2(0.f, 0.f);
     }
     if (MEANVAR) {
+        __syncthreads();
+        const int slab = threadIdx.x >> 5, row = threadIdx.x & 31;      // the CTA's two slabs
+        const int64_t first = (int64_t)blockIdx.x * WARPS + 4 * slab;
+        if (slab < WARPS / 4 && first < (M / QB) * per_row) {
+            float2 a = row_part[4 * slab][row];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            float a = ps[i], b2 = pq[i];
-#pragma unroll
-            for (int mask = 1; mask < 8; mask <<= 1) {
-                a = __fadd_rn(a, __shfl_xor_sync(0xffffffffu, a, mask));
-                b2 = __fadd_rn(b2, __shfl_xor_sync(0xffffffffu, b2, mask));
+            for (int k = 1; k < 4; ++k) {
+                const float2 b = row_part[4 * slab + k][row];
+                a.x = __fadd_rn(a.x, b.x); a.y = __fadd_rn(a.y, b.y);
             }
-            if (c == 0) {
-                const int64_t row = tm * QB + 4 * i + r;
-                part_sum[row * groups_n + grp] = a;
-                part_sq[row * groups_n + grp] = b2;
-            }
+            const int64_t slab_tm = (int64_t)((uint32_t)first / (uint32_t)per_row), grp = (int64_t)((uint32_t)first % (uint32_t)per_row) >> 2;
+            part_sum[(slab_tm * QB + row) * slabs_n + grp] = a.x;
+            part_sq[(slab_tm * QB + row) * slabs_n + grp] = a.y;
         }
     }
 }
 
 // mean = sum/N; rstd = 1/sqrt(sumsq/N - mean^2)
-__global__ void meanvar_finish_kernel(const float* __restrict__ part_sum, const float* __restrict__ part_sq, int64_t M, int64_t tiles_n,
+__global__ void meanvar_finish_kernel(const float* part_sum, const float* part_sq, int64_t M, int64_t tiles_n,
                                       int64_t N, float* __restrict__ mean, float* __restrict__ rstd) {
     const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    grid_dependency_wait();
     if (row >= M) return;
     float a = 0.f, b = 0.f;
     for (int64_t k = 0; k < tiles_n; ++k) {
@@ -1324,10 +1343,10 @@ static int ensure_gelu_table(cudaStream_t st, bool backward) {
 template <typename T>
 static void launch_add(const void* x1, const int8_t* q2, const __half* s2, int64_t M, int64_t N, float* y1, int8_t* qy, __half* sy,
                        float* ps, float* pq, bool meanvar, bool stochastic, SrCfg sr, cudaStream_t st) {
-    // work items: 32x32 blocks, or (with row statistics) 128-column slabs of four blocks walked by one warp each
+    // a warp per 32x32 block; with row statistics the blocks of a short last 128-column slab are padded to four
     const T* xp = (const T*)x1;
-    const int64_t blocks = (M / QB) * (N / QB), slabs = (M / QB) * ((N + 127) / 128);
-    const unsigned grid_b = (unsigned)((blocks + WARPS - 1) / WARPS), grid_s = (unsigned)((slabs + WARPS - 1) / WARPS);
+    const int64_t blocks = (M / QB) * (N / QB), padded = (M / QB) * 4 * ((N + 127) / 128);
+    const unsigned grid_b = (unsigned)((blocks + WARPS - 1) / WARPS), grid_s = (unsigned)((padded + WARPS - 1) / WARPS);
     if (meanvar) add_kernel<T, true, false><<<grid_s, THREADS, 0, st>>>(xp, q2, s2, M, N, y1, qy, sy, ps, pq, sr);
     else if (stochastic) add_kernel<T, false, true><<<grid_b, THREADS, 0, st>>>(xp, q2, s2, M, N, y1, qy, sy, ps, pq, sr);
     else add_kernel<T, false, false><<<grid_b, THREADS, 0, st>>>(xp, q2, s2, M, N, y1, qy, sy, ps, pq, sr);
@@ -1506,8 +1525,7 @@ static int add_impl(const void* x1, int x1_dtype, const int8_t* q2, const void* 
     }
     if (int e = check_launch()) return e;
     if (meanvar) {
-        meanvar_finish_kernel<<<(unsigned)((M + 127) / 128), 128, 0, st>>>(ps, pq, M, tiles_n, N, mean, rstd);
-        return check_launch();
+        return launch_dependent(meanvar_finish_kernel, (unsigned)((M + 63) / 64), 64, st, (const float*)ps, (const float*)pq, M, tiles_n, N, mean, rstd);
     }
     return JF_OK;
 }
