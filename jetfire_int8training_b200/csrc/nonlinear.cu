@@ -11,11 +11,14 @@
 //   * the re-quantising division is an exact IEEE quotient computed with a shared correctly-rounded reciprocal (fast path
 //     chosen once per warp), rounding is an add of 1.5*2^23, bytes are gathered with prmt;
 //   * int8 -> fp32 avoids the conversion unit (prmt into the mantissa of 2^23, one subtract).
-// Tile widths: 32 columns (at most 80 registers, three 8-warp CTAs per SM) for the kernels with arithmetic per element --
+// Tile widths: 32 columns (at most 80 registers, three or four 8-warp CTAs per SM) for the kernels with arithmetic per element --
 // quantize, GELU forward / backward, LayerNorm forward, the residual adds -- which is what keeps enough loads in flight;
-// 64 columns for the pure data movers (dequantize, transpose, quantize with the transposed copy).  LayerNorm backward and the
-// residual add with row statistics work on the reference's 128-column slab: two warps of 64 columns, resp. one warp walking
-// four 32-column tiles.
+// 64 columns for the pure data movers (dequantize, transpose, quantize with the transposed copy).  LayerNorm backward works on the
+// reference's 128-column slab with two warps of 64 columns.
+//
+// What bounds them.  Stochastic rounding: the generator's wide multiplications (4 clocks each on the FMA-heavy pipe), quantize + SR of
+// fp16 [12288 x 2304] 31.1 -> 27.9 us (3.0 TB/s, FMA-heavy pipe 60 %, ALU 56 %, issue slots 57 %); GELU backward + SR [12288 x 3072]
+// 57.4 -> 49.8 us; LayerNorm backward + SR [8192 x 1600] 33.4 -> 30.6 us; add + mean/var [3104 x 1600] 14.4 -> 10.2 us (4.0 TB/s).
 #include <mutex>
 #include <type_traits>
 
@@ -596,7 +599,7 @@ __device__ __forceinline__ TableRow load_table_row(const float2* table, __half s
 //   (2) table entries: lane l divides its eight exact y values (a = 4l+1 .. 4l+4, both signs) by the block scale -- the exact
 //       quotient is the Markstein sequence with the correctly rounded reciprocal, valid because scale32 >= 0.17/127;
 //   (3) a block of small inputs (absmax below 0.17, rare) finds its absmax over the elements and divides with div.rn.
-__global__ void __launch_bounds__(THREADS, 3)
+__global__ void __launch_bounds__(THREADS, 4)
 gelu_fwd_kernel(const int8_t* __restrict__ qx, const __half* __restrict__ sx, int64_t M, int64_t N, int8_t* __restrict__ qy,
                 __half* __restrict__ sy) {
     constexpr int TW = 32, NP = Geo<TW>::NP;
@@ -607,7 +610,8 @@ gelu_fwd_kernel(const int8_t* __restrict__ qx, const __half* __restrict__ sx, in
     float* ytab = ytab_all[warp];
     uint8_t* btab_g = btab_all[warp];
     const uint32_t btab = (uint32_t)__cvta_generic_to_shared(btab_g);
-    for_each_tile<TW, Raw, true>(
+    for_each_tile<TW, Raw, false>(        // four CTAs per SM hide the loads better than three with the next tile prefetched: 25.9 -> 25.1 us
+
         M, N,
         [&](const Tile& t, Raw& r) {
             load_rows<TW>(qx, t, N, r.d);
@@ -723,7 +727,8 @@ gelu_bwd_kernel(const int8_t* __restrict__ qx, const __half* __restrict__ sx, co
     using Raw = RawQ2<NP>;
     __shared__ __align__(16) float lut_all[WARPS][256];
     float* lut = lut_all[threadIdx.x >> 5];
-    for_each_tile<TW, Raw, true>(
+    for_each_tile<TW, Raw, false>(        // prefetching the next tile spills at 80 registers: 59.5 against 51.4 us on [12288 x 3072] with SR
+
         M, N,
         [&](const Tile& t, Raw& r) {
             load_rows<TW>(qx, t, N, r.a);
@@ -767,13 +772,14 @@ gelu_bwd_kernel(const int8_t* __restrict__ qx, const __half* __restrict__ sx, co
 // LayerNorm forward: y = ((fp16(q*s) - mean) * rstd) * gamma; statistics are inputs
 // =========================================================================================================
 template <int TW>
-__global__ void __launch_bounds__(THREADS, TW == 32 ? 3 : 2)
+__global__ void __launch_bounds__(THREADS, TW == 32 ? 4 : 2)
 ln_fwd_kernel(const int8_t* __restrict__ qx, const __half* __restrict__ sx, const float* __restrict__ gamma,
               const float* __restrict__ mean, const float* __restrict__ rstd, int64_t M, int64_t N, int8_t* __restrict__ qy,
               __half* __restrict__ sy) {
     constexpr int NP = Geo<TW>::NP;
     using Raw = RawQ<NP>;
-    for_each_tile<TW, Raw, true>(
+    for_each_tile<TW, Raw, false>(        // no prefetch, four CTAs per SM: [12288 x 768] 8.5 -> 7.5 us (2.5 TB/s; bound by instruction latencies)
+
         M, N,
         [&](const Tile& t, Raw& r) {
             load_rows<TW>(qx, t, N, r.d);
@@ -1448,7 +1454,7 @@ int jf_int8_gelu_forward(const int8_t* qx, const void* sx, int64_t M, int64_t N,
     JF_REQUIRE_ALIGNED(qx); JF_REQUIRE_ALIGNED(qy);
     cudaStream_t st = (cudaStream_t)stream;
     if (int e = ensure_gelu_table(st, false)) return e;
-    gelu_fwd_kernel<<<grid_for<32>(M, N, persistent_ctas(3)), THREADS, 0, st>>>(qx, (const __half*)sx, M, N, qy, (__half*)sy);
+    gelu_fwd_kernel<<<grid_for<32>(M, N, persistent_ctas(4)), THREADS, 0, st>>>(qx, (const __half*)sx, M, N, qy, (__half*)sy);
     return check_launch();
 }
 
@@ -1475,7 +1481,7 @@ int jf_int8_layernorm_forward(const int8_t* qx, const void* sx, const float* gam
     if (int e = check_mn(M, N)) return e;
     JF_REQUIRE_ALIGNED(qx); JF_REQUIRE_ALIGNED(qy); JF_REQUIRE_ALIGNED(gamma);
     cudaStream_t st = (cudaStream_t)stream;
-    ln_fwd_kernel<32><<<grid_for<32>(M, N, persistent_ctas(3)), THREADS, 0, st>>>(qx, (const __half*)sx, gamma, mean, rstd, M, N, qy, (__half*)sy);
+    ln_fwd_kernel<32><<<grid_for<32>(M, N, persistent_ctas(4)), THREADS, 0, st>>>(qx, (const __half*)sx, gamma, mean, rstd, M, N, qy, (__half*)sy);
     return check_launch();
 }
 

@@ -376,3 +376,24 @@ def test_errors(NL):
         NL.int8_quantize(torch.randn(48, 32, device=DEV), 32)          # rows not a multiple of 32
     with pytest.raises(ValueError):
         NL.int8_quantize(torch.randn(32, 32, device=DEV), 16)          # only QB = 32
+
+
+@pytest.mark.parametrize("M,N", [(32, 32), (32, 128), (64, 160), (96, 416), (992, 32), (256, 1600)])
+def test_row_statistics_and_gamma_partials_at_slab_edges(NL, oracle, M, N):
+    """Add + mean/var (four warps of a 128-column slab meet in shared memory, a short last slab has idle ones) and the dgamma reduction
+    (eight rows in flight, then a remainder: 1 to 31 partial rows)."""
+    g = torch.Generator().manual_seed(M + N)
+    x1 = torch.randn(M, N, generator=g)
+    q, s = oracle.int8_quantize(torch.randn(M, N, generator=g).numpy())
+    y1, y2, sy, mean, rstd = NL.int8_add_Ifp_Ig16_Ofp_Og_MeanVar(t(x1), t(q), t(s), 32)
+    y = n(y1).astype(np.float64)
+    assert np.array_equal(n(y1), x1.numpy() + q.astype(np.float32) * np.repeat(np.repeat(s.astype(np.float32), 32, 0), 32, 1))
+    np.testing.assert_allclose(n(mean), y.mean(1), rtol=1e-4, atol=1e-6)
+    np.testing.assert_allclose(n(rstd), 1 / np.sqrt((y * y).mean(1) - y.mean(1) ** 2), rtol=1e-4)
+    gq, gs = oracle.int8_quantize((1e-2 * torch.randn(M, N, generator=g)).numpy())
+    w = (1 + 0.1 * torch.randn(N, generator=g))
+    _, _, dw = NL.int8_layernorm_backward(t(q), t(s), t(gq), t(gs), t(w), 32, mean, rstd)
+    x = q.astype(np.float64) * np.repeat(np.repeat(s.astype(np.float64), 32, 0), 32, 1)
+    dy = gq.astype(np.float64) * np.repeat(np.repeat(gs.astype(np.float64), 32, 0), 32, 1)
+    want = (dy * (x - n(mean)[:, None]) * n(rstd)[:, None]).sum(0)
+    np.testing.assert_allclose(n(dw), want, rtol=2e-2, atol=2e-2 * np.abs(want).max())
