@@ -55,6 +55,11 @@ int jf_abi_version(void);
 int jf_int8_quantize(const void* x, int x_dtype, int64_t M, int64_t N, int8_t* q, void* s, int8_t* qt,
                      int stochastic, const float* noise, uint64_t seed, uint64_t offset, void* stream);
 
+/* Quantise a tensor that is given as `count` (1..4) column parts [M, cols] lying apart: the result of jf_int8_quantize on their
+ * concatenation [M, count * cols], without the concatenation. */
+int jf_int8_quantize_parts(int count, const void* const* x, int x_dtype, int64_t M, int64_t cols, int8_t* q, void* s, int stochastic,
+                           uint64_t seed, uint64_t offset, void* stream);
+
 /* The same round-to-nearest quantisation for up to 8 tensors of one dtype in one launch: x[j] is [M[j], N[j]], q[j] / s[j] its payload
  * and scales.  For the weight matrices a caller quantises at the start of every forward pass (INT8_GPT2/qmodel.py:92, 139, 199-200:
  * four int8_quantize calls per transformer block); results are identical to `count` calls of jf_int8_quantize.  `x`, `M`, `N`, `q`, `s`
@@ -109,6 +114,12 @@ int jf_int8_add(const void* x1, int x1_dtype, const int8_t* q2, const void* s2, 
  * scratch: fp32 [2 * M * ceil(N/128)] workspace for the per-tile row partial sums. */
 int jf_int8_add_meanvar(const void* x1, int x1_dtype, const int8_t* q2, const void* s2, int64_t M, int64_t N, float* y1,
                         int8_t* qy, void* sy, float* mean, float* rstd, float* scratch, void* stream);
+
+/* Residual add with y1 as fp32 or (y1_dtype JF_BF16) rounded once to bf16; payload, scales and statistics are those of the fp32 sum. */
+int jf_int8_add_out(const void* x1, int x1_dtype, const int8_t* q2, const void* s2, int64_t M, int64_t N, void* y1, int y1_dtype,
+                    int8_t* qy, void* sy, int stochastic, const float* noise, uint64_t seed, uint64_t offset, void* stream);
+int jf_int8_add_meanvar_out(const void* x1, int x1_dtype, const int8_t* q2, const void* s2, int64_t M, int64_t N, void* y1, int y1_dtype,
+                            int8_t* qy, void* sy, float* mean, float* rstd, float* scratch, void* stream);
 
 /* Allocation-free variant of jf_int8_add_meanvar.  It has no counterpart in the reference.
  * For hosts that cannot hand the library a workspace (a plug-in interface that passes only inputs and outputs, a runtime
@@ -206,6 +217,12 @@ int jf_lm_loss_forward(const void* logits_bf16, const int64_t* targets, int64_t 
                        void* stream);
 int jf_lm_loss_backward(void* logits_bf16, const int64_t* targets, const float* lse, const float* grad_out, float inv_count,
                         int64_t rows, int64_t V, void* stream);
+
+/* The same with the mean taken on the device: *mean = mean loss over the positions that count, *count = their number (at least 1); the backward pass divides by that number. */
+int jf_lm_loss_forward_mean(const void* logits_bf16, const int64_t* targets, int64_t rows, int64_t V, float* lse, float* loss_rows,
+                            float* mean, float* count, void* stream);
+int jf_lm_loss_backward_mean(void* logits_bf16, const int64_t* targets, const float* lse, const float* grad_out, const float* count,
+                             int64_t rows, int64_t V, void* stream);
 
 /* ------------------------------------------------------------------------------------------------------------
  * Optimiser step of the caller (the un-quantised tail):  scaler.unscale_(optimizer); clip_grad_norm_(params, max_norm);

@@ -20,9 +20,9 @@ from .. import rng
 from .._lib import host
 
 __all__ = [
-    "int8_quantize", "int8_quantize_many", "int8_quantize_transpose", "int8_transpose", "int8_dequantize",
+    "int8_quantize", "int8_quantize_many", "int8_quantize_parts", "int8_quantize_transpose", "int8_transpose", "int8_dequantize",
     "int8_gelu_forward", "int8_gelu_backward", "int8_layernorm_forward", "int8_layernorm_backward",
-    "int8_add_Ifp_Ig16_Ofp_Og", "int8_add_Ifp_Ig16_Ofp_Og_MeanVar", "set_sr_noise",
+    "int8_add_Ifp_Ig16_Ofp_Og", "int8_add_Ifp_Ig16_Ofp_Og_MeanVar", "int8_add_out", "set_sr_noise",
 ]
 
 _SR_NOISE = "philox"
@@ -65,6 +65,15 @@ def int8_quantize_many(tensors, QB):
     199-200).  Returns [(q, scale), ...], bit-identical to int8_quantize on each tensor."""
     _qb(QB)
     return host().quantize_many(tensors)
+
+
+def int8_quantize_parts(parts, QB, stochastic=False, *, sr_key=None):
+    """int8_quantize of torch.cat(parts, -1) for one to four parts of one shape and dtype, without the concatenation (the gradients of
+    Q, K and V in front of the QKV projection's backward pass)."""
+    _qb(QB)
+    if stochastic and sr_key is None and _SR_NOISE == "torch":
+        return int8_quantize(torch.cat(tuple(parts), dim=-1), QB, stochastic=True)
+    return host().quantize_parts(parts, stochastic, *_sr(stochastic, None, sr_key, parts[0]))
 
 
 def int8_quantize_transpose(x, QB, stochastic=False, transpose_output_2d=False, *, noise=None, sr_key=None):
@@ -114,10 +123,21 @@ def int8_layernorm_backward(x, sx, g, sg, w, QB, m, v, stochastic=False, eps=1e-
 def int8_add_Ifp_Ig16_Ofp_Og(x1, x2, s_x2, QB, stochastic=False, *, noise=None, sr_key=None):
     """Jetfire/Nonlinear/add.py:164-211.  Returns (y1 fp32, y2 int8, s_y2 fp16)."""
     _qb(QB)
-    return host().add(x1, x2, s_x2, False, stochastic, *_sr(stochastic, noise, sr_key, x1))
+    return host().add(x1, x2, s_x2, False, False, stochastic, *_sr(stochastic, noise, sr_key, x1))
 
 
 def int8_add_Ifp_Ig16_Ofp_Og_MeanVar(x1, x2, s_x2, QB):
     """Jetfire/Nonlinear/add_mean_var.py:179-231.  Returns (y1 fp32, y2 int8, s_y2 fp16, mean, rstd)."""
     _qb(QB)
-    return host().add(x1, x2, s_x2, True, False, None, 0, 0)
+    return host().add(x1, x2, s_x2, True, False, False, None, 0, 0)
+
+
+def int8_add_out(x1, x2, s_x2, QB, out_dtype, mean_var=False, stochastic=False, *, sr_key=None):
+    """The residual adds with y1 in `out_dtype` (fp32, or bf16 rounded once from the fp32 sum): int8_add_Ifp_Ig16_Ofp_Og or, with
+    mean_var, int8_add_Ifp_Ig16_Ofp_Og_MeanVar, followed by y1.to(out_dtype) -- in one pass."""
+    _qb(QB)
+    if out_dtype not in (torch.float32, torch.bfloat16):
+        raise TypeError("int8_add_out writes fp32 or bf16")
+    if mean_var and stochastic:
+        raise ValueError("the add with row statistics rounds to nearest")
+    return host().add(x1, x2, s_x2, mean_var, out_dtype == torch.bfloat16, stochastic, *_sr(stochastic, None, sr_key, x1))

@@ -15,7 +15,7 @@ HOST = os.path.join(HERE, "_host_ops.so")
 SOURCES = ["nonlinear.cu", "gemm.cu", "noalloc.cu", "lm_loss.cu", "optim.cu"]
 HOST_SOURCES = ["host_ops.cpp"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-              "-Xcompiler", "-fPIC", "-shared"]
+              "-Xcompiler", "-fPIC", "-shared", "--threads", "0"]
 
 
 def _sources():

@@ -303,23 +303,17 @@ static int device_info(DeviceInfo** out) {
 
 #include "gemm_launch.inc"
 
-// Number of K ranges of a weight-gradient GEMM.  An SM works through ceil(items / SMs) items, two at a time (one alone reaches ~0.7 of
-// their common rate); an item costs its K blocks (~0.11 us each) plus ~7 K blocks' worth of start and epilogue; a split adds a kernel and
-// the fp32 partials' way through memory (~4 TB/s: they are mostly served by L2).  Ranges keep at least 16 K blocks.
-// [768 x 2304], K = 12288: 216 tiles leave a quarter of the 296 CTA slots idle; two ranges take 76 instead of 92 us.
+// Number of K ranges of a weight-gradient GEMM.  It fixes the order in which dW is summed, hence its bits, and stochastic rounding turns a
+// last-bit difference in the weights into percents of the next step's gradients: the plan therefore stays the one of 128 x 128 tiles, one
+// per SM, although the CTAs are 128 x 64.  (A plan that counts rounds of CTA slots gives [768 x 2304], K = 12288 two ranges: 76 us, not 92.)
 static int plan_splits(int64_t M, int64_t N, int64_t K, int split_k, int sm_count, int64_t* per_out) {
     const int64_t nkb = K / QB;
     int64_t s = split_k;
     if (s <= 0) {
-        const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-        double best = 0.0;
-        s = 1;
-        for (int64_t c = 1; c <= 8 && (c == 1 || nkb / c >= 16); ++c) {
-            const int64_t per = (nkb + c - 1) / c, rounds = (tiles * c + sm_count - 1) / sm_count;
-            double cost = (double)rounds * (double)(per + 7) * (rounds == 1 ? 1.4 : 1.0);
-            if (c > 1) cost += (3.0 + (double)c * (double)M * (double)N * 8.0 / 4e6) / 0.11;
-            if (c == 1 || cost < best) { best = cost; s = c; }
-        }
+        s = sm_count / (((M + 127) / 128) * ((N + 127) / 128));
+        const int64_t cap = nkb / 16;   // keep at least 16 K blocks per range
+        if (s > cap) s = cap;
+        if (s < 1) s = 1;
     }
     if (s > nkb) s = nkb;
     const int64_t per = (nkb + s - 1) / s;

@@ -47,6 +47,7 @@ __device__ __forceinline__ void block_lse(float& m, float& s) {
 __global__ void __launch_bounds__(LM_THREADS) lm_loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const int64_t* __restrict__ targets,
                                                                 int64_t V, float* __restrict__ lse, float* __restrict__ loss) {
     const int64_t row = blockIdx.x;
+    grid_launch_dependents();      // the mean over the rows, where it follows
     const __nv_bfloat16* x = logits + row * V;
     float m = -INFINITY, s = 0.f;
     const int64_t chunks = V / 8;
@@ -79,12 +80,13 @@ __global__ void __launch_bounds__(LM_THREADS) lm_loss_fwd_kernel(const __nv_bflo
 // in place: logits[row, c] <- (exp(logits[row, c] - lse[row]) - [c == target]) * (*grad_out) * inv_count   (0 for an ignored row)
 __global__ void __launch_bounds__(LM_THREADS) lm_loss_bwd_kernel(__nv_bfloat16* __restrict__ logits, const int64_t* __restrict__ targets,
                                                                 const float* __restrict__ lse, const float* __restrict__ grad_out,
-                                                                float inv_count, int64_t V) {
+                                                                const float* __restrict__ count, float inv_count, int64_t V) {
     const int64_t row = blockIdx.x;
     __nv_bfloat16* x = logits + row * V;
     const int64_t t = targets[row];
     const bool live = t >= 0 && t < V;
-    const float scale = live ? __ldg(grad_out) * inv_count : 0.f;
+    // the mean's gradient: upstream / (number of counted positions), from device memory when the host does not know the number
+    const float scale = live ? (count ? __fdiv_rn(__ldg(grad_out), __ldg(count)) : __ldg(grad_out)) * inv_count : 0.f;
     const float l2 = lse[row] * 1.4426950408889634f;
     const int64_t chunks = V / 8;
     for (int64_t c = threadIdx.x; c < chunks; c += LM_THREADS) {
@@ -112,6 +114,32 @@ __global__ void __launch_bounds__(LM_THREADS) lm_loss_bwd_kernel(__nv_bfloat16* 
     }
 }
 
+// mean = sum(loss) / count, count = number of targets in [0, V), at least 1.  One CTA: a few thousand values.
+__global__ void __launch_bounds__(1024) lm_loss_mean_kernel(const float* loss, const int64_t* __restrict__ targets, int64_t rows, int64_t V, float* __restrict__ mean,
+                                                            float* __restrict__ count) {
+    __shared__ float ssum[32];
+    __shared__ int scnt[32];
+    grid_dependency_wait();
+    float a = 0.f;
+    int n = 0;
+    for (int64_t r = threadIdx.x; r < rows; r += 1024) {
+        a += loss[r];
+        const int64_t t = __ldg(targets + r);
+        n += (t >= 0 && t < V) ? 1 : 0;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) { a += __shfl_xor_sync(0xffffffffu, a, o); n += __shfl_xor_sync(0xffffffffu, n, o); }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (lane == 0) { ssum[warp] = a; scnt[warp] = n; }
+    __syncthreads();
+    if (warp == 0) {
+        a = ssum[lane]; n = scnt[lane];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) { a += __shfl_xor_sync(0xffffffffu, a, o); n += __shfl_xor_sync(0xffffffffu, n, o); }
+        if (lane == 0) { const float c = (float)max(n, 1); *mean = __fdiv_rn(a, c); *count = c; }
+    }
+}
+
 }  // namespace jf
 
 using namespace jf;
@@ -127,13 +155,30 @@ int jf_lm_loss_forward(const void* logits_bf16, const int64_t* targets, int64_t 
     return check_launch();
 }
 
-int jf_lm_loss_backward(void* logits_bf16, const int64_t* targets, const float* lse, const float* grad_out, float inv_count,
-                        int64_t rows, int64_t V, void* stream) {
+int jf_lm_loss_forward_mean(const void* logits_bf16, const int64_t* targets, int64_t rows, int64_t V, float* lse, float* loss_rows, float* mean,
+                            float* count, void* stream) {
+    if (!mean || !count) return JF_ERR_NULL;
+    if (int e = jf_lm_loss_forward(logits_bf16, targets, rows, V, lse, loss_rows, stream)) return e;
+    return launch_dependent(lm_loss_mean_kernel, 1, 1024, (cudaStream_t)stream, (const float*)loss_rows, targets, rows, V, mean, count);
+}
+
+static int lm_loss_backward(void* logits_bf16, const int64_t* targets, const float* lse, const float* grad_out, const float* count, float inv_count,
+                            int64_t rows, int64_t V, void* stream) {
     if (!logits_bf16 || !targets || !lse || !grad_out) return JF_ERR_NULL;
     if (rows <= 0 || V <= 0 || rows >= (int64_t(1) << 31)) return JF_ERR_SHAPE;
     if (!aligned16(logits_bf16) || (V % 8 != 0 && rows > 1)) return JF_ERR_ALIGN;
-    lm_loss_bwd_kernel<<<(unsigned)rows, LM_THREADS, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)logits_bf16, targets, lse, grad_out, inv_count, V);
+    lm_loss_bwd_kernel<<<(unsigned)rows, LM_THREADS, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)logits_bf16, targets, lse, grad_out, count, inv_count, V);
     return check_launch();
+}
+
+int jf_lm_loss_backward(void* logits_bf16, const int64_t* targets, const float* lse, const float* grad_out, float inv_count, int64_t rows, int64_t V,
+                        void* stream) {
+    return lm_loss_backward(logits_bf16, targets, lse, grad_out, nullptr, inv_count, rows, V, stream);
+}
+int jf_lm_loss_backward_mean(void* logits_bf16, const int64_t* targets, const float* lse, const float* grad_out, const float* count, int64_t rows,
+                             int64_t V, void* stream) {
+    if (!count) return JF_ERR_NULL;
+    return lm_loss_backward(logits_bf16, targets, lse, grad_out, count, 1.0f, rows, V, stream);
 }
 
 }  // extern "C"

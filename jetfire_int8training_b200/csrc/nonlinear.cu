@@ -355,11 +355,25 @@ __device__ __forceinline__ void load_rows(const int8_t* q, const Tile& t, int64_
 __device__ __forceinline__ __half load_scale16(const __half* s, const Tile& t, int64_t N) {
     return t.active ? __ldg(s + t.tm * (N / QB) + (t.col >> 5)) : __float2half_rn(0.f);
 }
-template <typename T, int TW>
-__device__ __forceinline__ void load_x(const T* x, const Tile& t, int64_t N, RawX<T, Geo<TW>::NP>& r) {
+// A tensor given as column parts [M, cols] that lie apart (the gradients of Q, K and V): part p holds columns p * cols ..
+constexpr int QPARTS_MAX = 4;
+template <typename T>
+struct Parts {
+    const T* p[QPARTS_MAX];
+    int64_t cols;
+};
+template <typename T>
+__device__ __forceinline__ const T* row_chunk(const T* x, int64_t row, int64_t col, int64_t N) { return x + row * N + col; }
+template <typename T>
+__device__ __forceinline__ const T* row_chunk(const Parts<T>& x, int64_t row, int64_t col, int64_t) {
+    const uint32_t part = (uint32_t)col / (uint32_t)x.cols;
+    return x.p[part] + row * x.cols + (col - (int64_t)part * x.cols);
+}
+template <typename T, int TW, class Src>
+__device__ __forceinline__ void load_x(const Src& x, const Tile& t, int64_t N, RawX<T, Geo<TW>::NP>& r) {
 #pragma unroll
     for (int i = 0; i < Geo<TW>::NP; ++i) {
-        const uint4* p4 = reinterpret_cast<const uint4*>(x + row_of<TW>(t, i) * N + t.col);
+        const uint4* p4 = reinterpret_cast<const uint4*>(row_chunk(x, row_of<TW>(t, i), t.active ? t.col : 0, N));
 #pragma unroll
         for (int k = 0; k < (int)sizeof(T); ++k) r.d[i][k] = t.active ? __ldg(p4 + k) : make_uint4(0, 0, 0, 0);
     }
@@ -422,9 +436,9 @@ __device__ __forceinline__ float absmax16(const uint4 (&d)[2], __nv_bfloat16) {
 // quantize / quantize_transpose.  The tile stays packed in registers; it is widened once for the block absmax and once more
 // for the quantisation, which is cheaper than holding 64 fp32 values next to the prefetched next tile.
 // =========================================================================================================
-template <typename T, int TW, bool SR, bool TRANSPOSE>
+template <typename T, int TW, bool SR, bool TRANSPOSE, class Src = const T*>
 __global__ void __launch_bounds__(THREADS, TW == 32 ? 3 : 2)
-quantize_kernel(const T* __restrict__ x, int64_t M, int64_t N, int8_t* __restrict__ q, __half* __restrict__ s,
+quantize_kernel(const Src x, int64_t M, int64_t N, int8_t* __restrict__ q, __half* __restrict__ s,
                 int8_t* __restrict__ qt, SrCfg sr) {
     constexpr int NP = Geo<TW>::NP;
     using Raw = RawX<T, NP>;
@@ -432,7 +446,7 @@ quantize_kernel(const T* __restrict__ x, int64_t M, int64_t N, int8_t* __restric
     uint32_t* tile_words = TRANSPOSE ? smem_tiles + (threadIdx.x >> 5) * 8 * TW : nullptr;
     // fp32 input: the packed tile is already 64 registers, prefetching a second one would spill
     for_each_tile<TW, Raw, sizeof(T) != 4>(
-        M, N, [&](const Tile& t, Raw& r) { load_x<T, TW>(x, t, N, r); },
+        M, N, [&](const Tile& t, Raw& r) { load_x<T, TW, Src>(x, t, N, r); },
         [&](const Tile& t, Raw& r) {
             float m = 0.f;
 #pragma unroll
@@ -1157,27 +1171,22 @@ __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bfloat16* p) {
                        __uint_as_float(v.y & 0xFFFF0000u));
 }
 
-// Sum of eight per-lane values over the eight lanes of a row group: lane c ends with the total of value c.  Seven shuffles (the halves of
-// the value list are exchanged, then quarters, then eighths) instead of three per value.
-__device__ __forceinline__ float rowgroup_sum8(float (&v)[8], int c) {
-#pragma unroll
-    for (int mask = 4; mask >= 1; mask >>= 1)
-#pragma unroll
-        for (int k = 0; k < mask; ++k) {
-            const bool up = c & mask;                     // keep the upper half of the list
-            const float send = up ? v[k] : v[k + mask], keep = up ? v[k + mask] : v[k];
-            v[k] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, mask));
-        }
-    return v[0];
+// the residual stream leaves as fp32, or rounded once to bf16 for a caller that would narrow it (statistics and payload are of the fp32 sum)
+__device__ __forceinline__ void store4(float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void store4(__nv_bfloat16* p, const float4& v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
 
-template <typename T, bool MEANVAR, bool SR>
+template <typename T, typename OutT, bool MEANVAR, bool SR>
 __global__ void __launch_bounds__(THREADS, 3)
 add_kernel(const T* __restrict__ x1, const int8_t* __restrict__ q2, const __half* __restrict__ s2, int64_t M, int64_t N,
-           float* __restrict__ y1, int8_t* __restrict__ qy, __half* __restrict__ sy, float* __restrict__ part_sum,
+           OutT* __restrict__ y1, int8_t* __restrict__ qy, __half* __restrict__ sy, float* __restrict__ part_sum,
            float* __restrict__ part_sq, SrCfg sr) {
-    // Row statistics: the four warps of a 128-column slab leave their blocks' row sums in shared memory and are summed in column order.
-    __shared__ float2 row_part[MEANVAR ? WARPS : 1][MEANVAR ? QB : 1];
+    // Row statistics: the four warps of a 128-column slab leave each lane's sums (of its four columns of a row) in shared memory.  They are
+    // added per lane in column order and then over the eight lanes as a tree -- the order of one warp that walks the four blocks, so that
+    // mean and rstd, which decide roundings of everything behind them, do not depend on how the work is split.
+    __shared__ float row_sum[MEANVAR ? WARPS : 1][MEANVAR ? 256 : 1], row_sq[MEANVAR ? WARPS : 1][MEANVAR ? 256 : 1];   // [warp][8 row + lane]
     if (MEANVAR) grid_launch_dependents();                    // the statistics' last step
     const int64_t blocks_n = N / QB;                          // blocks per row of blocks
     const int64_t slabs_n = (blocks_n + 3) / 4;               // MEANVAR: warps are numbered by slab, a short last slab leaves some idle
@@ -1198,43 +1207,47 @@ add_kernel(const T* __restrict__ x1, const int8_t* __restrict__ q2, const __half
         for (int i = 0; i < 8; ++i) v[i] = load4<T>(x1 + base + (int64_t)(4 * i) * N);
         const float sc = __half2float(__ldg(s2 + tm * blocks_n + tn));
         float m = 0.f;
-        float ps[8], pq[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             v[i].x = __fadd_rn(v[i].x, __fmul_rn(byte_to_float(qw[i], 0), sc));
             v[i].y = __fadd_rn(v[i].y, __fmul_rn(byte_to_float(qw[i], 1), sc));
             v[i].z = __fadd_rn(v[i].z, __fmul_rn(byte_to_float(qw[i], 2), sc));
             v[i].w = __fadd_rn(v[i].w, __fmul_rn(byte_to_float(qw[i], 3), sc));
-            *reinterpret_cast<float4*>(y1 + base + (int64_t)(4 * i) * N) = v[i];
+            store4(y1 + base + (int64_t)(4 * i) * N, v[i]);
             m = fmaxf(fmaxf(m, fmaxf(fabsf(v[i].x), fabsf(v[i].y))), fmaxf(fabsf(v[i].z), fabsf(v[i].w)));
             if (MEANVAR) {
-                ps[i] = __fadd_rn(__fadd_rn(v[i].x, v[i].y), __fadd_rn(v[i].z, v[i].w));
-                pq[i] = __fadd_rn(__fadd_rn(__fmul_rn(v[i].x, v[i].x), __fmul_rn(v[i].y, v[i].y)),
-                                  __fadd_rn(__fmul_rn(v[i].z, v[i].z), __fmul_rn(v[i].w, v[i].w)));
+                row_sum[warp][32 * i + lane] = __fadd_rn(__fadd_rn(v[i].x, v[i].y), __fadd_rn(v[i].z, v[i].w));      // row 4 i + r, lane c
+                row_sq[warp][32 * i + lane] = __fadd_rn(__fadd_rn(__fmul_rn(v[i].x, v[i].x), __fmul_rn(v[i].y, v[i].y)),
+                                                        __fadd_rn(__fmul_rn(v[i].z, v[i].z), __fmul_rn(v[i].w, v[i].w)));
             }
         }
         const float amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
         const float scale32 = __fdiv_rn(amax, 127.0f);
-        if (MEANVAR) row_part[warp][4 * c + r] = make_float2(rowgroup_sum8(ps, c), rowgroup_sum8(pq, c));   // row 4 i + r, i = c
         emit_block4<true, SR>([&](int i) { return v[i]; }, scale32, base, N, c, qy, sr);
         if (lane == 0) sy[tm * blocks_n + tn] = __float2half_rn(scale32);
     } else if (MEANVAR) {
-        row_part[warp][lane] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) row_sum[warp][32 * i + lane] = row_sq[warp][32 * i + lane] = 0.f;
     }
     if (MEANVAR) {
         __syncthreads();
-        const int slab = threadIdx.x >> 5, row = threadIdx.x & 31;      // the CTA's two slabs
-        const int64_t first = (int64_t)blockIdx.x * WARPS + 4 * slab;
-        if (slab < WARPS / 4 && first < (M / QB) * per_row) {
-            float2 a = row_part[4 * slab][row];
+        const int k = threadIdx.x, row = k >> 3;                       // thread = (row of the slab, lane of the row)
 #pragma unroll
-            for (int k = 1; k < 4; ++k) {
-                const float2 b = row_part[4 * slab + k][row];
-                a.x = __fadd_rn(a.x, b.x); a.y = __fadd_rn(a.y, b.y);
+        for (int slab = 0; slab < WARPS / 4; ++slab) {                 // the CTA's two slabs
+            const int64_t first = (int64_t)blockIdx.x * WARPS + 4 * slab;
+            float a = row_sum[4 * slab][k], b = row_sq[4 * slab][k];
+#pragma unroll
+            for (int w = 1; w < 4; ++w) { a = __fadd_rn(a, row_sum[4 * slab + w][k]); b = __fadd_rn(b, row_sq[4 * slab + w][k]); }
+#pragma unroll
+            for (int mask = 1; mask < 8; mask <<= 1) {
+                a = __fadd_rn(a, __shfl_xor_sync(0xffffffffu, a, mask));
+                b = __fadd_rn(b, __shfl_xor_sync(0xffffffffu, b, mask));
             }
-            const int64_t slab_tm = (int64_t)((uint32_t)first / (uint32_t)per_row), grp = (int64_t)((uint32_t)first % (uint32_t)per_row) >> 2;
-            part_sum[(slab_tm * QB + row) * slabs_n + grp] = a.x;
-            part_sq[(slab_tm * QB + row) * slabs_n + grp] = a.y;
+            if ((k & 7) == 0 && first < (M / QB) * per_row) {
+                const int64_t slab_tm = (int64_t)((uint32_t)first / (uint32_t)per_row), grp = (int64_t)((uint32_t)first % (uint32_t)per_row) >> 2;
+                part_sum[(slab_tm * QB + row) * slabs_n + grp] = a;
+                part_sq[(slab_tm * QB + row) * slabs_n + grp] = b;
+            }
         }
     }
 }
@@ -1346,16 +1359,17 @@ static int ensure_gelu_table(cudaStream_t st, bool backward) {
     return cudaStreamWaitEvent(st, ts.ready, 0) == cudaSuccess ? JF_OK : JF_ERR_LAUNCH;
 }
 
-template <typename T>
-static void launch_add(const void* x1, const int8_t* q2, const __half* s2, int64_t M, int64_t N, float* y1, int8_t* qy, __half* sy,
+template <typename T, typename OutT>
+static void launch_add(const void* x1, const int8_t* q2, const __half* s2, int64_t M, int64_t N, void* y1, int8_t* qy, __half* sy,
                        float* ps, float* pq, bool meanvar, bool stochastic, SrCfg sr, cudaStream_t st) {
     // a warp per 32x32 block; with row statistics the blocks of a short last 128-column slab are padded to four
     const T* xp = (const T*)x1;
+    OutT* yp = (OutT*)y1;
     const int64_t blocks = (M / QB) * (N / QB), padded = (M / QB) * 4 * ((N + 127) / 128);
     const unsigned grid_b = (unsigned)((blocks + WARPS - 1) / WARPS), grid_s = (unsigned)((padded + WARPS - 1) / WARPS);
-    if (meanvar) add_kernel<T, true, false><<<grid_s, THREADS, 0, st>>>(xp, q2, s2, M, N, y1, qy, sy, ps, pq, sr);
-    else if (stochastic) add_kernel<T, false, true><<<grid_b, THREADS, 0, st>>>(xp, q2, s2, M, N, y1, qy, sy, ps, pq, sr);
-    else add_kernel<T, false, false><<<grid_b, THREADS, 0, st>>>(xp, q2, s2, M, N, y1, qy, sy, ps, pq, sr);
+    if (meanvar) add_kernel<T, OutT, true, false><<<grid_s, THREADS, 0, st>>>(xp, q2, s2, M, N, yp, qy, sy, ps, pq, sr);
+    else if (stochastic) add_kernel<T, OutT, false, true><<<grid_b, THREADS, 0, st>>>(xp, q2, s2, M, N, yp, qy, sy, ps, pq, sr);
+    else add_kernel<T, OutT, false, false><<<grid_b, THREADS, 0, st>>>(xp, q2, s2, M, N, yp, qy, sy, ps, pq, sr);
 }
 
 extern "C" {
@@ -1391,6 +1405,34 @@ int jf_int8_quantize(const void* x, int x_dtype, int64_t M, int64_t N, int8_t* q
         case JF_F32: launch_quantize<float>(x, M, N, q, sh, qt, sto, sr, st); break;
         case JF_F16: launch_quantize<__half>(x, M, N, q, sh, qt, sto, sr, st); break;
         case JF_BF16: launch_quantize<__nv_bfloat16>(x, M, N, q, sh, qt, sto, sr, st); break;
+        default: return JF_ERR_DTYPE;
+    }
+    return check_launch();
+}
+
+int jf_int8_quantize_parts(int count, const void* const* x, int x_dtype, int64_t M, int64_t cols, int8_t* q, void* s, int stochastic, uint64_t seed,
+                           uint64_t offset, void* stream) {
+    if (count <= 0 || count > QPARTS_MAX) return JF_ERR_ARG;
+    JF_REQUIRE_PTR(x); JF_REQUIRE_PTR(q); JF_REQUIRE_PTR(s);
+    if (!mult32(cols) || cols >= (int64_t(1) << 28)) return JF_ERR_SHAPE;
+    const int64_t N = count * cols;
+    if (int e = check_mn(M, N)) return e;
+    for (int k = 0; k < count; ++k) { JF_REQUIRE_PTR(x[k]); JF_REQUIRE_ALIGNED(x[k]); }
+    JF_REQUIRE_ALIGNED(q);
+    const SrCfg sr = make_sr(nullptr, seed, offset, M, N);
+    auto launch = [&](auto in) {
+        using T = decltype(in);
+        Parts<T> p{};
+        for (int k = 0; k < count; ++k) p.p[k] = (const T*)x[k];
+        p.cols = cols;
+        const unsigned grid = grid_for<32>(M, N, persistent_ctas(3));
+        if (stochastic) quantize_kernel<T, 32, true, false, Parts<T>><<<grid, THREADS, 0, (cudaStream_t)stream>>>(p, M, N, q, (__half*)s, nullptr, sr);
+        else quantize_kernel<T, 32, false, false, Parts<T>><<<grid, THREADS, 0, (cudaStream_t)stream>>>(p, M, N, q, (__half*)s, nullptr, sr);
+    };
+    switch (x_dtype) {
+        case JF_F32: launch(float()); break;
+        case JF_F16: launch(__half()); break;
+        case JF_BF16: launch(__nv_bfloat16()); break;
         default: return JF_ERR_DTYPE;
     }
     return check_launch();
@@ -1507,7 +1549,7 @@ int jf_int8_layernorm_backward(const int8_t* qx, const void* sx, const int8_t* q
     return launch_dependent(ln_bwd_dw_kernel, (unsigned)((N + 31) / 32), 256, st, (const float*)scratch, M / QB, N, dgamma);
 }
 
-static int add_impl(const void* x1, int x1_dtype, const int8_t* q2, const void* s2, int64_t M, int64_t N, float* y1, int8_t* qy,
+static int add_impl(const void* x1, int x1_dtype, const int8_t* q2, const void* s2, int64_t M, int64_t N, void* y1, int y1_dtype, int8_t* qy,
                     void* sy, float* mean, float* rstd, float* scratch, bool meanvar, bool stochastic, SrCfg sr, cudaStream_t st) {
     JF_REQUIRE_PTR(x1); JF_REQUIRE_PTR(q2); JF_REQUIRE_PTR(s2); JF_REQUIRE_PTR(y1); JF_REQUIRE_PTR(qy); JF_REQUIRE_PTR(sy);
     if (int e = check_mn(M, N)) return e;
@@ -1523,10 +1565,16 @@ static int add_impl(const void* x1, int x1_dtype, const int8_t* q2, const void* 
     }
     const __half* s2h = (const __half*)s2;
     __half* syh = (__half*)sy;
+    if (y1_dtype != JF_F32 && y1_dtype != JF_BF16) return JF_ERR_DTYPE;
+    auto launch = [&](auto in) {
+        using T = decltype(in);
+        if (y1_dtype == JF_F32) launch_add<T, float>(x1, q2, s2h, M, N, y1, qy, syh, ps, pq, meanvar, stochastic, sr, st);
+        else launch_add<T, __nv_bfloat16>(x1, q2, s2h, M, N, y1, qy, syh, ps, pq, meanvar, stochastic, sr, st);
+    };
     switch (x1_dtype) {
-        case JF_F32: launch_add<float>(x1, q2, s2h, M, N, y1, qy, syh, ps, pq, meanvar, stochastic, sr, st); break;
-        case JF_F16: launch_add<__half>(x1, q2, s2h, M, N, y1, qy, syh, ps, pq, meanvar, stochastic, sr, st); break;
-        case JF_BF16: launch_add<__nv_bfloat16>(x1, q2, s2h, M, N, y1, qy, syh, ps, pq, meanvar, stochastic, sr, st); break;
+        case JF_F32: launch(float()); break;
+        case JF_F16: launch(__half()); break;
+        case JF_BF16: launch(__nv_bfloat16()); break;
         default: return JF_ERR_DTYPE;
     }
     if (int e = check_launch()) return e;
@@ -1536,16 +1584,24 @@ static int add_impl(const void* x1, int x1_dtype, const int8_t* q2, const void* 
     return JF_OK;
 }
 
+int jf_int8_add_out(const void* x1, int x1_dtype, const int8_t* q2, const void* s2, int64_t M, int64_t N, void* y1, int y1_dtype, int8_t* qy,
+                    void* sy, int stochastic, const float* noise, uint64_t seed, uint64_t offset, void* stream) {
+    SrCfg sr = make_sr(noise, seed, offset, M, N);
+    return add_impl(x1, x1_dtype, q2, s2, M, N, y1, y1_dtype, qy, sy, nullptr, nullptr, nullptr, false, stochastic != 0, sr, (cudaStream_t)stream);
+}
 int jf_int8_add(const void* x1, int x1_dtype, const int8_t* q2, const void* s2, int64_t M, int64_t N, float* y1, int8_t* qy, void* sy,
                 int stochastic, const float* noise, uint64_t seed, uint64_t offset, void* stream) {
-    SrCfg sr = make_sr(noise, seed, offset, M, N);
-    return add_impl(x1, x1_dtype, q2, s2, M, N, y1, qy, sy, nullptr, nullptr, nullptr, false, stochastic != 0, sr, (cudaStream_t)stream);
+    return jf_int8_add_out(x1, x1_dtype, q2, s2, M, N, y1, JF_F32, qy, sy, stochastic, noise, seed, offset, stream);
 }
 
+int jf_int8_add_meanvar_out(const void* x1, int x1_dtype, const int8_t* q2, const void* s2, int64_t M, int64_t N, void* y1, int y1_dtype,
+                            int8_t* qy, void* sy, float* mean, float* rstd, float* scratch, void* stream) {
+    SrCfg sr{};
+    return add_impl(x1, x1_dtype, q2, s2, M, N, y1, y1_dtype, qy, sy, mean, rstd, scratch, true, false, sr, (cudaStream_t)stream);
+}
 int jf_int8_add_meanvar(const void* x1, int x1_dtype, const int8_t* q2, const void* s2, int64_t M, int64_t N, float* y1, int8_t* qy,
                         void* sy, float* mean, float* rstd, float* scratch, void* stream) {
-    SrCfg sr{};
-    return add_impl(x1, x1_dtype, q2, s2, M, N, y1, qy, sy, mean, rstd, scratch, true, false, sr, (cudaStream_t)stream);
+    return jf_int8_add_meanvar_out(x1, x1_dtype, q2, s2, M, N, y1, JF_F32, qy, sy, mean, rstd, scratch, stream);
 }
 
 }  // extern "C"

@@ -12,6 +12,7 @@ Differences from the reference's module, none of which touch the operators' sema
 (the reference's fp16 overflows under its 2^24 loss scale), the materialised dY^T copies are not made (the GEMMs read dY
 in place), and the weight matrices are quantised eight per kernel launch at the start of the forward pass.
 """
+import contextlib
 import math
 from dataclasses import dataclass
 
@@ -21,6 +22,7 @@ from torch.nn import functional as F
 
 from . import Linear as L
 from . import Nonlinear as NL
+from ._lib import host
 from .lm_loss import lm_cross_entropy
 
 QB = 32
@@ -67,102 +69,156 @@ def _i8(t):
     return t.view(torch.int8)
 
 
-class _Begin(torch.autograd.Function):
-    """Entry of the INT8 stream: quantise the embedding output (reference: QModel_bgn_func, qmodel.py:309-326)."""
+# A model's pass is one autograd node per part: embedding, each block, the final LayerNorm, the LM head.  With a node for each group of
+# operators and torch's views, splits and casts between them, a 2-layer 256-wide model spent 2.3 ms per step on the host around 0.6 ms of
+# device work, and GPT-2 124M ~0.7 ms on narrowing copies of the residual stream and concatenations of the QKV gradient.  A node per block (not one for all) keeps the gradients of a block available to DDP while the earlier ones run.
+
+
+def _add(x1, q, s, dtype, mean_var=False, stochastic=False):
+    """Residual add whose fp output the residual stream carries in `dtype` (an operator module without the one-pass form: add, then cast)."""
+    fused = getattr(NL, "int8_add_out", None)
+    if fused is not None:
+        return fused(x1, q, s, QB, dtype, mean_var=mean_var, stochastic=stochastic)
+    if mean_var:
+        y, *rest = NL.int8_add_Ifp_Ig16_Ofp_Og_MeanVar(x1, q, s, QB)
+    else:
+        y, *rest = NL.int8_add_Ifp_Ig16_Ofp_Og(x1, q, s, QB, stochastic=stochastic)
+    return (y.to(dtype), *rest)
+
+
+def _quantise_parts(parts):
+    """Stochastically rounded block quantisation of the concatenated parts."""
+    fused = getattr(NL, "int8_quantize_parts", None)
+    if fused is not None:
+        return fused(parts, QB, stochastic=True)
+    return NL.int8_quantize(torch.cat(parts, dim=-1), QB, stochastic=True)
+
+
+def _attention(qkv, n_head):
+    B, T, C = qkv.shape[0], qkv.shape[1], qkv.shape[2] // 3
+    q, k, v = [t.view(B, T, n_head, C // n_head).transpose(1, 2) for t in qkv.split(C, dim=2)]
+    return F.scaled_dot_product_attention(q, k, v, is_causal=True).transpose(1, 2).contiguous().view(B, T, C)
+
+
+class _Embed(torch.autograd.Function):
+    """Token + position embedding and the entry of the INT8 stream: quantise their sum, row mean and 1 / std (reference:
+    QModel_bgn_func, qmodel.py:309-326).  `tied` carries the LM head's gradient of the shared token matrix from the head's backward
+    pass, which always runs first, so that the two are added without a widened copy of either."""
 
     @staticmethod
-    def forward(ctx, x):
+    def forward(ctx, idx, wte, wpe, tied):
+        x, mean, rstd = host().embed_forward(idx, wte, wpe)
         qx, sx = NL.int8_quantize(x, QB)
-        return x, _f8(qx), sx
+        ctx.save_for_backward(idx)
+        ctx.sizes, ctx.tied = (wte.shape[0], wpe.shape[0]), tied
+        ctx.set_materialize_grads(False)
+        ctx.mark_non_differentiable(mean, rstd)
+        return x, _f8(qx), sx, mean, rstd
 
     @staticmethod
-    def backward(ctx, g, qg, sg):
-        return g
+    def backward(ctx, g, qg, sg, _m, _r):
+        idx, = ctx.saved_tensors
+        dwte, dwpe = host().embed_backward(idx, g, ctx.tied.pop("dw", None), *ctx.sizes)
+        return None, dwte, dwpe, None
 
 
-class _End(torch.autograd.Function):
-    """Exit of the INT8 stream: in the backward pass the incoming fp gradient is block-quantised with stochastic rounding and
-    seeds the INT8 gradient stream (reference: QModel_end_func, qmodel.py:343-362)."""
+class _Block(torch.autograd.Function):
+    """One transformer block, forward and backward over the operators (reference: _QAttentionPart1 / _QAttentionPart2 / _QMLPResidual,
+    qmodel.py:86-267): LayerNorm + QKV projection (dequantised fp16) -> attention -> quantise -> output projection + residual add with row
+    statistics -> LayerNorm + FC1 + GELU + FC2 + residual add with row statistics.  In the backward pass the gradient travels as (fp
+    residual gradient in the residual's type, int8 payload, scales)."""
 
     @staticmethod
-    def forward(ctx, x, qx, sx):
-        return x.clone()
+    def forward(ctx, x, qx, sx, mean, rstd, ln1, w_qkv, w_proj, ln2, w1, w2, n_head):
+        qx = _i8(qx)
+        (qwq, swq), (qwp, swp), (qw1, sw1), (qw2, sw2) = [quantized_weight(w) for w in (w_qkv, w_proj, w1, w2)]
+        qn, sn, _ = NL.int8_layernorm_forward(qx, sx, ln1, mean, rstd, QB)
+        qkv = L.int8_linear_forward(qn, sn, qwq, swq, False, QB)
+        fused = host().attention_forward(qkv, n_head)
+        if fused is not None:
+            y, max_q, max_k, *att = fused
+            ctx.graph = None
+        else:                                        # another attention backend: through its own autograd graph
+            with torch.enable_grad():
+                leaf = qkv.detach().requires_grad_()
+                out = _attention(leaf, n_head)
+            y, max_q, max_k, att = out.detach(), 0, 0, []
+            ctx.graph = (leaf, out)
+        qy, sy = NL.int8_quantize(y, QB)
+        qo, so = L.int8_linear_forward(qy, sy, qwp, swp, True, QB)
+        x1, qx1, sx1, mean1, rstd1 = NL.int8_add_Ifp_Ig16_Ofp_Og_MeanVar(x.contiguous(), qo, so, QB)
+        qn1, sn1, _ = NL.int8_layernorm_forward(qx1, sx1, ln2, mean1, rstd1, QB)
+        qh, sh = L.int8_linear_forward(qn1, sn1, qw1, sw1, True, QB)
+        qa, sa = NL.int8_gelu_forward(qh, sh, QB)
+        qo, so = L.int8_linear_forward(qa, sa, qw2, sw2, True, QB)
+        x2, qx2, sx2, mean2, rstd2 = _add(x1, qo, so, torch.bfloat16, mean_var=True)
+        ctx.save_for_backward(qx, sx, mean, rstd, ln1, qn, sn, qwq, swq, qkv, qy, sy, qwp, swp, qx1, sx1, mean1, rstd1, ln2, qn1, sn1, qw1, sw1,
+                              qh, sh, qa, sa, qw2, sw2, *att)
+        ctx.meta = (n_head, max_q, max_k, x.dtype)
+        ctx.set_materialize_grads(False)
+        ctx.mark_non_differentiable(mean2, rstd2)
+        return x2, _f8(qx2), sx2, mean2, rstd2
+
+    @staticmethod
+    def backward(ctx, fpg, qg, sg, _m, _r):
+        (qx, sx, mean, rstd, ln1, qn, sn, qwq, swq, qkv, qy, sy, qwp, swp, qx1, sx1, mean1, rstd1, ln2, qn1, sn1, qw1, sw1,
+         qh, sh, qa, sa, qw2, sw2, *att) = ctx.saved_tensors
+        n_head, max_q, max_k, dtype = ctx.meta
+        qg, sg, dw2 = _linear_backward(qa, sa, _i8(qg), sg, qw2, sw2)
+        qg, sg = NL.int8_gelu_backward(qh, sh, qg, sg, QB, stochastic=True)
+        qg, sg, dw1 = _linear_backward(qn1, sn1, qg, sg, qw1, sw1)
+        qg, sg, dln2 = NL.int8_layernorm_backward(qx1, sx1, qg, sg, ln2, QB, mean1, rstd1, stochastic=True)
+        fpg, qg, sg = _add(fpg.contiguous(), qg, sg, dtype, stochastic=True)
+        g16, dwp = _linear_backward(qy, sy, qg, sg, qwp, swp, dgrad_quantize=False)
+        if ctx.graph is None:
+            gq, gk, gv = host().attention_backward(g16, qkv, n_head, max_q, max_k, *att)
+            qg, sg = _quantise_parts([gq, gk, gv])
+        else:
+            leaf, out = ctx.graph
+            gqkv, = torch.autograd.grad(out, leaf, g16, retain_graph=True)
+            qg, sg = NL.int8_quantize(gqkv.contiguous(), QB, stochastic=True)
+        qg, sg, dwq = _linear_backward(qn, sn, qg, sg, qwq, swq)
+        qg, sg, dln1 = NL.int8_layernorm_backward(qx, sx, qg, sg, ln1, QB, mean, rstd, stochastic=True)
+        fpg, qg, sg = _add(fpg, qg, sg, dtype, stochastic=True)
+        return fpg, _f8(qg), sg, None, None, dln1, dwq, dwp, dln2, dw1, dw2, None
+
+
+class _Final(torch.autograd.Function):
+    """Exit of the INT8 stream and final LayerNorm, whose bf16 output is what the LM head reads: in the backward pass the fp gradient is
+    block-quantised with stochastic rounding and seeds the INT8 gradient stream (reference: QModel_end_func, qmodel.py:343-362)."""
+
+    @staticmethod
+    def forward(ctx, x, qx, sx, ln_f):
+        y, xf, mean, rstd = host().final_norm_forward(x, ln_f, 1e-5)
+        ctx.save_for_backward(xf, ln_f, mean, rstd)
+        ctx.narrow = x.dtype == torch.bfloat16
+        return y
+
+    @staticmethod
+    def backward(ctx, gy):
+        xf, ln_f, mean, rstd = ctx.saved_tensors
+        g, dln = host().final_norm_backward(gy, xf, ln_f, mean, rstd, ctx.narrow)
+        qg, sg = NL.int8_quantize(g, QB, stochastic=True)
+        return g, _f8(qg), sg, dln
+
+
+class _Head(torch.autograd.Function):
+    """LM head: bf16 logits = x W^T on the shared token matrix.  Its bf16 weight gradient is handed to _Embed's backward pass through
+    `tied`."""
+
+    @staticmethod
+    def forward(ctx, x, wte, tied):
+        x2, w = x.reshape(-1, x.shape[-1]), wte.to(torch.bfloat16)
+        ctx.save_for_backward(x2, w)
+        ctx.shape, ctx.tied = x.shape, tied
+        return torch.mm(x2, w.t()).view(*x.shape[:-1], w.shape[0])
 
     @staticmethod
     def backward(ctx, g):
-        g = g.contiguous()
-        qg, sg = NL.int8_quantize(g, QB, stochastic=True)
-        return g, _f8(qg), sg
-
-
-class _AttnIn(torch.autograd.Function):
-    """LayerNorm + QKV projection (reference: _QAttentionPart1, qmodel.py:86-132).  Output: dequantised fp16 QKV."""
-
-    @staticmethod
-    def forward(ctx, residual, qx, sx, w_qkv, ln_w, mean, rstd):
-        qx = _i8(qx)
-        qw, sw = quantized_weight(w_qkv)
-        qn, sn, _ = NL.int8_layernorm_forward(qx, sx, ln_w, mean, rstd, QB)
-        y = L.int8_linear_forward(qn, sn, qw, sw, False, QB)
-        ctx.save_for_backward(qx, sx, qn, sn, qw, sw, ln_w, mean, rstd)
-        return residual, y
-
-    @staticmethod
-    def backward(ctx, fpg, g):
-        qx, sx, qn, sn, qw, sw, ln_w, mean, rstd = ctx.saved_tensors
-        qg, sg = NL.int8_quantize(g.contiguous(), QB, stochastic=True)
-        qg, sg, dw = _linear_backward(qn, sn, qg, sg, qw, sw)
-        qg, sg, dln = NL.int8_layernorm_backward(qx, sx, qg, sg, ln_w, QB, mean, rstd, stochastic=True)
-        res_g, qg, sg = NL.int8_add_Ifp_Ig16_Ofp_Og(fpg.contiguous(), qg, sg, QB, stochastic=True)
-        return res_g, _f8(qg), sg, dw, dln, None, None
-
-
-class _AttnOut(torch.autograd.Function):
-    """Attention output projection + residual add with row statistics (reference: _QAttentionPart2, qmodel.py:134-170)."""
-
-    @staticmethod
-    def forward(ctx, residual, y, w_proj):
-        qw, sw = quantized_weight(w_proj)
-        qy, sy = NL.int8_quantize(y.contiguous(), QB)
-        qo, so = L.int8_linear_forward(qy, sy, qw, sw, True, QB)
-        fpx, qx, sx, mean, rstd = NL.int8_add_Ifp_Ig16_Ofp_Og_MeanVar(residual.contiguous(), qo, so, QB)
-        ctx.save_for_backward(qy, sy, qw, sw)
-        ctx.mark_non_differentiable(mean, rstd)
-        return fpx, _f8(qx), sx, mean, rstd
-
-    @staticmethod
-    def backward(ctx, fpg, qg, sg, _m, _r):
-        qy, sy, qw, sw = ctx.saved_tensors
-        g16, dw = _linear_backward(qy, sy, _i8(qg), sg, qw, sw, dgrad_quantize=False)
-        return fpg, g16, dw
-
-
-class _MLP(torch.autograd.Function):
-    """LayerNorm + FC1 + GELU + FC2 + residual add with row statistics (reference: _QMLPResidual, qmodel.py:190-267)."""
-
-    @staticmethod
-    def forward(ctx, residual, qx, sx, w1, w2, ln_w, mean, rstd):
-        qx = _i8(qx)
-        qw1, sw1 = quantized_weight(w1)
-        qw2, sw2 = quantized_weight(w2)
-        qn, sn, _ = NL.int8_layernorm_forward(qx, sx, ln_w, mean, rstd, QB)
-        qh, sh = L.int8_linear_forward(qn, sn, qw1, sw1, True, QB)
-        qa, sa = NL.int8_gelu_forward(qh, sh, QB)
-        qo, so = L.int8_linear_forward(qa, sa, qw2, sw2, True, QB)
-        fpx, qy, sy, mean2, rstd2 = NL.int8_add_Ifp_Ig16_Ofp_Og_MeanVar(residual.contiguous(), qo, so, QB)
-        ctx.save_for_backward(qx, sx, qn, sn, qh, sh, qa, sa, qw1, sw1, qw2, sw2, ln_w, mean, rstd)
-        ctx.mark_non_differentiable(mean2, rstd2)
-        return fpx.to(torch.bfloat16), _f8(qy), sy, mean2, rstd2
-
-    @staticmethod
-    def backward(ctx, fpg, qg, sg, _m, _r):
-        qx, sx, qn, sn, qh, sh, qa, sa, qw1, sw1, qw2, sw2, ln_w, mean, rstd = ctx.saved_tensors
-        qg, sg, dw2 = _linear_backward(qa, sa, _i8(qg), sg, qw2, sw2)
-        qg, sg = NL.int8_gelu_backward(qh, sh, qg, sg, QB, stochastic=True)
-        qg, sg, dw1 = _linear_backward(qn, sn, qg, sg, qw1, sw1)
-        qg, sg, dln = NL.int8_layernorm_backward(qx, sx, qg, sg, ln_w, QB, mean, rstd, stochastic=True)
-        res_g, qg, sg = NL.int8_add_Ifp_Ig16_Ofp_Og(fpg.contiguous(), qg, sg, QB, stochastic=True)
-        return res_g, _f8(qg), sg, dw1, dw2, dln, None, None
+        x2, w = ctx.saved_tensors
+        g2 = g.reshape(-1, w.shape[0]).to(torch.bfloat16)
+        ctx.tied["dw"] = torch.mm(g2.t(), x2)
+        return torch.mm(g2, w).view(ctx.shape), None, None
 
 
 def _linear_backward(qx, sx, qg, sg, qw, sw, dgrad_quantize=True):
@@ -184,17 +240,7 @@ class Block(nn.Module):
         self.c_proj2 = nn.Parameter(torch.empty(C, 4 * C))
 
     def forward(self, x, qx, sx, mean, rstd):
-        B, T, C = x.shape
-        residual, qkv = _AttnIn.apply(x, qx, sx, self.c_attn, self.ln_1, mean, rstd)
-        q, k, v = qkv.split(C, dim=2)
-        hs = C // self.n_head
-        q = q.view(B, T, self.n_head, hs).transpose(1, 2)
-        k = k.view(B, T, self.n_head, hs).transpose(1, 2)
-        v = v.view(B, T, self.n_head, hs).transpose(1, 2)
-        y = F.scaled_dot_product_attention(q, k, v, is_causal=True)
-        y = y.transpose(1, 2).contiguous().view(B, T, C)
-        x, qx, sx, mean, rstd = _AttnOut.apply(residual, y, self.c_proj)
-        return _MLP.apply(x, qx, sx, self.c_fc, self.c_proj2, self.ln_2, mean, rstd)
+        return _Block.apply(x, qx, sx, mean, rstd, self.ln_1, self.c_attn, self.c_proj, self.ln_2, self.c_fc, self.c_proj2, self.n_head)
 
 
 class QGPT(nn.Module):
@@ -220,17 +266,12 @@ class QGPT(nn.Module):
     def forward(self, idx, targets, reuse_quantised_weights=False):
         """`reuse_quantised_weights`: the weights have not changed since the previous forward pass (micro-steps 2.. of a
         gradient-accumulation step), keep their quantisations."""
-        B, T = idx.shape
-        pos = torch.arange(T, device=idx.device)
-        x = self.wte(idx) + self.wpe(pos)
         quantise_weights([w for b in self.blocks for w in (b.c_attn, b.c_proj, b.c_fc, b.c_proj2)], reuse=reuse_quantised_weights)
-        x, qx, sx = _Begin.apply(x)
-        mean = x.mean(-1)
-        rstd = 1.0 / x.var(-1).sqrt()
-        for blk in self.blocks:
-            x, qx, sx, mean, rstd = blk(x, qx, sx, mean.detach(), rstd.detach())
-        x = _End.apply(x, qx, sx)
-        x = F.layer_norm(x.float(), (self.cfg.n_embd,), self.ln_f, None, 1e-5)
-        with torch.autocast("cuda", dtype=torch.bfloat16):
-            logits = F.linear(x, self.wte.weight)
+        tied = {}
+        with torch.autocast("cuda", enabled=False) if torch.is_autocast_enabled("cuda") else contextlib.nullcontext():
+            state = _Embed.apply(idx, self.wte.weight, self.wpe.weight, tied)
+            for blk in self.blocks:
+                state = blk(*state)
+            x, qx, sx, _, _ = state
+            logits = _Head.apply(_Final.apply(x, qx, sx, self.ln_f), self.wte.weight, tied)
         return lm_cross_entropy(logits, targets)       # no fp32 copy of the [tokens, vocab] logits; gradient written in place

@@ -8,7 +8,7 @@ is ever allocated.  There is no CPU path.
 """
 import torch
 
-from ._lib import lib, check
+from ._lib import host
 
 __all__ = ["lm_cross_entropy"]
 
@@ -16,33 +16,15 @@ __all__ = ["lm_cross_entropy"]
 class _LMLoss(torch.autograd.Function):
     @staticmethod
     def forward(ctx, logits, targets):
-        if not logits.is_cuda:
-            raise RuntimeError("jetfire_int8training_b200 operators need CUDA tensors (there is no CPU path)")
-        if logits.dtype != torch.bfloat16:
-            raise TypeError("lm_cross_entropy takes bf16 logits")
-        V = logits.shape[-1]
-        x = logits.reshape(-1, V)
-        if not x.is_contiguous():
-            x = x.contiguous()
-        t = targets.reshape(-1).to(torch.int64).contiguous()
-        rows = x.shape[0]
-        lse = torch.empty(rows, dtype=torch.float32, device=x.device)
-        loss_rows = torch.empty(rows, dtype=torch.float32, device=x.device)
-        st = torch.cuda.current_stream().cuda_stream
-        check(lib().jf_lm_loss_forward(x.data_ptr(), t.data_ptr(), rows, V, lse.data_ptr(), loss_rows.data_ptr(), st), "lm_cross_entropy")
-        count = ((t >= 0) & (t < V)).sum().clamp(min=1).to(torch.float32)
+        loss, x, t, lse, count = host().lm_loss_forward(logits, targets)
         ctx.save_for_backward(x, t, lse, count)
         ctx.shape = logits.shape
-        return loss_rows.sum() / count
+        return loss
 
     @staticmethod
     def backward(ctx, grad_out):
         x, t, lse, count = ctx.saved_tensors
-        rows, V = x.shape
-        g = (grad_out.to(torch.float32) / count).reshape(1).contiguous()
-        st = torch.cuda.current_stream().cuda_stream
-        check(lib().jf_lm_loss_backward(x.data_ptr(), t.data_ptr(), lse.data_ptr(), g.data_ptr(), 1.0, rows, V, st),
-              "lm_cross_entropy(backward)")
+        host().lm_loss_backward(grad_out, x, t, lse, count)
         return x.view(ctx.shape), None
 
 

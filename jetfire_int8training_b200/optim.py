@@ -13,7 +13,7 @@ import math
 
 import torch
 
-from ._lib import lib, check
+from ._lib import check, host, lib
 
 
 class ClipAdamW:
@@ -60,14 +60,17 @@ class ClipAdamW:
         self._starts = (ctypes.c_int64 * n)(*starts)
         self._wd = (ctypes.c_float * n)(*wds)
         self._partial = torch.empty(c, dtype=torch.float32, device=dev)
-        self._GradArray = ctypes.c_void_p * n
         # [scale, steps since the scale changed, optimiser steps taken, norm, applied factor, skipped, 2 x scratch]
         self.state = torch.zeros(8, dtype=torch.float32, device=dev)
         self.state[0] = 1.0 if loss_scale is None else float(loss_scale)
+        # what every step passes on, once: views and addresses of the buffers that live as long as this object
+        self._scale, self._result = self.state[0], self.state[3:6]       # [gradient norm, applied factor, skipped]
+        self._buffers = (self.flat.data_ptr(), self.exp_avg.data_ptr(), self.exp_avg_sq.data_ptr())
+        self._state_ptr, self._partial_ptr = self.state.data_ptr(), self._partial.data_ptr()
 
     def scale_loss(self, loss):
         """loss x current loss scale (a device-side multiplication); call backward() on the result."""
-        return loss * self.state[0]
+        return loss * self._scale
 
     @property
     def step_count(self):
@@ -79,24 +82,14 @@ class ClipAdamW:
         return buf[s: s + self.params[i].numel()].view(self.params[i].shape)
 
     def step(self):
-        grads = []
-        for p in self.params:
-            g = p.grad
-            if g is None:
-                raise RuntimeError("ClipAdamW.step(): a parameter has no gradient")
-            if g.dtype != torch.float32 or not g.is_contiguous():
-                g = g.float().contiguous()
-                p.grad = g
-            grads.append(g)
-        check(lib().jf_adamw_clip_step(len(self.params), self._GradArray(*[g.data_ptr() for g in grads]), self._numel, self._starts,
-                                       self._wd, self.flat.data_ptr(), self.exp_avg.data_ptr(), self.exp_avg_sq.data_ptr(),
-                                       self.total_chunks, self.lr, self.betas[0], self.betas[1], self.eps, self.max_norm,
-                                       self.state.data_ptr(), self.growth_interval, self.growth_factor, self.backoff_factor,
-                                       self._partial.data_ptr(), torch.cuda.current_stream().cuda_stream), "adamw_clip_step")
-        out = self.state[3:6].clone()          # [gradient norm, applied factor, skipped]
+        grads = host().gradient_pointers(self.params)
+        check(lib().jf_adamw_clip_step(len(self.params), grads, self._numel, self._starts, self._wd, *self._buffers, self.total_chunks, self.lr,
+                                       *self.betas, self.eps, self.max_norm, self._state_ptr, self.growth_interval, self.growth_factor,
+                                       self.backoff_factor, self._partial_ptr, torch.cuda.current_stream().cuda_stream), "adamw_clip_step")
+        out = self._result.clone()
         # the parameters were updated in place through the flat buffer by a kernel autograd does not know about: advance their
         # version counters (what an in-place torch operation would have done)
-        torch.autograd.graph.increment_version(self.params)
+        host().bump_versions(self.params)
         return out
 
     def zero_grad(self, set_to_none=True):
