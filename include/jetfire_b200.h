@@ -224,6 +224,10 @@ int jf_lm_loss_forward_mean(const void* logits_bf16, const int64_t* targets, int
 int jf_lm_loss_backward_mean(void* logits_bf16, const int64_t* targets, const float* lse, const float* grad_out, const float* count,
                              int64_t rows, int64_t V, void* stream);
 
+/* dst[i] += src[i] widened to fp32, i < n (a multiple of 8; both 16-byte aligned): the two gradients of a token matrix that is shared by the
+ * embedding and the LM head. */
+int jf_add_widened(float* dst, const void* src_bf16, int64_t n, void* stream);
+
 /* ------------------------------------------------------------------------------------------------------------
  * Optimiser step of the caller (the un-quantised tail):  scaler.unscale_(optimizer); clip_grad_norm_(params, max_norm);
  * scaler.step(optimizer); scaler.update()  of INT8_GPT2/train.py:320-329 (AdamW, torch's GradScaler), as one entry point that reads

@@ -41,6 +41,7 @@ SIGNATURES = {
     "jf_igemm_error_flag": ([], _int),
     "jf_lm_loss_forward": ([_vp, _vp, _i64, _i64, _vp, _vp, _vp], _int),
     "jf_lm_loss_backward": ([_vp, _vp, _vp, _vp, ctypes.c_float, _i64, _i64, _vp], _int),
+    "jf_add_widened": ([_vp, _vp, _i64, _vp], _int),
     "jf_lm_loss_forward_mean": ([_vp, _vp, _i64, _i64, _vp, _vp, _vp, _vp, _vp], _int),
     "jf_lm_loss_backward_mean": ([_vp, _vp, _vp, _vp, _vp, _i64, _i64, _vp], _int),
     "jf_int8_quantize_parts": ([_int, _vp, _int, _i64, _i64, _vp, _vp, _int, _u64, _u64, _vp], _int),

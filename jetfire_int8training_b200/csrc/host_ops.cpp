@@ -527,11 +527,13 @@ PyObject* embed_backward(PyObject* const* a) {
     const Tensor head = tensor_or_undefined(a[2]);
     const int64_t V = int_arg(a[3]), P = int_arg(a[4]);
     Tensor dwte, dwpe;
+    int added = JF_OK;
     {
         NoGil no_gil;
         Plain plain;
         dwte = at::embedding_dense_backward(g, idx, V, -1, false);
-        if (head.defined()) dwte.add_(head);
+        if (head.defined() && (dwte.numel() % 8 || !dwte.is_contiguous() || !head.is_contiguous() || head.scalar_type() != at::kBFloat16)) dwte.add_(head);
+        else if (head.defined()) added = jf_add_widened(dwte.mutable_data_ptr<float>(), head.const_data_ptr(), dwte.numel(), stream());
         dwpe = g.sum(0);
         if (idx.size(1) < P) {
             Tensor all = at::zeros({P, g.size(2)}, g.options());
@@ -539,6 +541,7 @@ PyObject* embed_backward(PyObject* const* a) {
             dwpe = all;
         }
     }
+    check(added, "embed_backward");
     return tuple(std::move(dwte), std::move(dwpe));
 }
 

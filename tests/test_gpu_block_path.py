@@ -111,3 +111,27 @@ def test_model_runs_through_another_attention_backend():
     for n in out[0][1]:
         a, b = out[0][1][n].flatten(), out[1][1][n].flatten()
         assert float(torch.dot(a, b) / (a.norm() * b.norm())) > 0.99, n
+
+
+@pytest.mark.parametrize("n", [8, 2040, 2048, 2056, 512 * 1000])
+def test_add_widened(n):
+    """Edges of a thread's eight elements and of a block's 2048."""
+    from jetfire_int8training_b200._lib import lib
+    g = _gen(n)
+    a, b = torch.randn(n + 8, generator=g, device=DEV), torch.randn(n, generator=g, device=DEV).bfloat16()
+    want = a.clone()
+    want[:n] += b.float()
+    assert lib().jf_add_widened(a.data_ptr(), b.data_ptr(), n, torch.cuda.current_stream().cuda_stream) == 0
+    assert torch.equal(a, want)
+    assert lib().jf_add_widened(a.data_ptr(), b.data_ptr(), n + 1, None) == -2
+
+
+@pytest.mark.parametrize("V", [8, 4088, 16376, 16384, 16392, 32776])
+def test_lm_loss_at_the_unrolled_step(V):
+    """Vocabularies around one and several steps of four 16-byte chunks per thread."""
+    from jetfire_int8training_b200.lm_loss import lm_cross_entropy
+    g = _gen(V)
+    x = (3 * torch.randn(5, V, generator=g, device=DEV)).bfloat16()
+    t = torch.tensor([0, V - 1, V // 2, -1, 1], device=DEV)
+    want = F.cross_entropy(x.float(), t, ignore_index=-1)
+    assert abs(float(lm_cross_entropy(x.clone(), t)) - float(want)) <= 1e-5 * abs(float(want))
