@@ -226,8 +226,7 @@ __device__ __forceinline__ void store_block(const GemmParams& p, const uint64_t 
 // out[i] = ((p0[i] + p1[i]) + p2[i]) + ...   then converted to the output type
 template <typename OutT>
 __global__ void splitk_reduce_kernel(const float* partials, int64_t splits, int64_t count, OutT* __restrict__ out) {
-    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
-    grid_dependency_wait();
+    const int64_t i = ((int64_t)(blockIdx.x + grid_dependency()) * blockDim.x + threadIdx.x) * 4;
     if (i >= count) return;
     float4 a = *reinterpret_cast<const float4*>(partials + i);
     for (int64_t k = 1; k < splits; ++k) {
@@ -426,8 +425,9 @@ int jf_igemm_wgrad(const int8_t* g, int g_transposed, const int8_t* x, const voi
     if (int e = launch()) return e;
     const int64_t count = M * N;
     const unsigned grid = (unsigned)((count / 4 + 255) / 256);
-    if (out_dtype == JF_F16) return launch_dependent(splitk_reduce_kernel<__half>, grid, 256, st, (const float*)scratch, (int64_t)splits, count, (__half*)dw);
-    return launch_dependent(splitk_reduce_kernel<float>, grid, 256, st, (const float*)scratch, (int64_t)splits, count, (float*)dw);
+    if (out_dtype == JF_F16) jf::launch(splitk_reduce_kernel<__half>, grid, 256, 0, st, scratch, splits, count, (__half*)dw);
+    else jf::launch(splitk_reduce_kernel<float>, grid, 256, 0, st, scratch, splits, count, (float*)dw);
+    return check_launch();
 }
 
 int jf_igemm_int32(const int8_t* a, const int8_t* b, int64_t M, int64_t N, int64_t K, int32_t* c, void* stream) {

@@ -6,7 +6,7 @@
 //
 // Two CTAs share an SM.  One CTA of 16 consumer warps per SM moves in step: all its warps leave the same barrier, load the same
 // accumulator and then queue for the same pipe, and nothing computes during an epilogue.  Two independent CTAs of 128 x 64 tiles with
-// eight consumer warps each fill one another's gaps: 12288 x 3072 x 768 forward 131 -> 111 us (520 TOPS), both gradients of 7392 x 1600 x 1600 227 -> 154 us.
+// eight consumer warps each fill one another's gaps: 12288 x 3072 x 768 forward 131 -> 111 us (520 TOPS), both gradients of 7392 x 1600 x 1600 227 -> 158 us.
 // Their operand traffic (12 KB per block product and SM; TMA delivers 56 B per clock and SM from L2) stays below the arithmetic.
 // Copying the operands to fp16 first (kind::f16 delivers floats, no conversion) is no way around it: at 16 KB per block product the
 // loads alone take 290 clocks, and the copies cost as much as they save at the layer shapes; at 8192^3 that kernel drew 1725 MHz from the
@@ -84,7 +84,6 @@ __device__ __forceinline__ bool lean_wait(uint64_t* bar, uint32_t parity, volati
 template <bool A_MN, bool B_MN, int CONV>
 __global__ void __launch_bounds__(GEMM_THREADS, 2)
 gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
-    grid_launch_dependents();      // the split-K reduction, where there is one
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     // barriers: pair_full[2] at 0, pair_empty[2] at 16, abort flag at 32, tmem slot at 36, drain at 40, full[STAGES] at 48,
@@ -114,6 +113,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    const uint32_t block_x = blockIdx.x + grid_dependency();      // barriers and tensor memory are set up while the previous kernel ends
     const uint32_t num_tiles = (uint32_t)(p.tiles_m * p.tiles_n), num_items = num_tiles * (uint32_t)p.splits;
     const int nkb = (int)p.nkb, per = (int)p.kb_per_split;
 
@@ -122,7 +122,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         if (ptx::elect_one()) {
             uint32_t it = 0, s = 0, ph = 0;
             bool ok = true;
-            for (uint32_t item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+            for (uint32_t item = block_x; item < num_items && ok; item += gridDim.x) {
                 const uint32_t tile = item % num_tiles, split = item / num_tiles;
                 int tm, tn;
                 tile_coords(tile, (uint32_t)p.tiles_m, (uint32_t)p.tiles_n, tm, tn);
@@ -150,7 +150,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         const uint64_t da_base = ptx::make_smem_desc_sw128(ptx::smem_u32(smem), A_MN ? 128 * 128 : 16, 1024);
         const uint64_t db_base = B_MN ? ptx::make_smem_desc_sw64(ptx::smem_u32(smem + A_BYTES), 128 * 64, 512)
                                       : ptx::make_smem_desc_sw128(ptx::smem_u32(smem + A_BYTES), 16, 1024);
-        for (uint32_t item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+        for (uint32_t item = block_x; item < num_items && ok; item += gridDim.x) {
             const uint32_t split = item / num_tiles;
             const int kb0 = (int)split * per, kb1 = min(nkb, kb0 + per);
             for (int kb = kb0; kb < kb1 && ok; kb += KB_PER_STAGE) {
@@ -187,7 +187,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         const uint32_t base = ptx::smem_u32(bars);
         const uint32_t t0 = tmem_base + ((uint32_t)(quad * 32) << 16) + cg * 32;
         uint32_t par = 0;
-        for (uint32_t item = blockIdx.x; item < num_items; item += gridDim.x) {
+        for (uint32_t item = block_x; item < num_items; item += gridDim.x) {
             const uint32_t tile = item % num_tiles, split = item / num_tiles;
             int tm, tn;
             tile_coords(tile, (uint32_t)p.tiles_m, (uint32_t)p.tiles_n, tm, tn);

@@ -24,28 +24,33 @@ inline int check_launch() {
     }
     return JF_OK;
 }
-// The second kernel of a reduction: it is launched while the first one, which has said grid_launch_dependents(), still runs, and waits for
-// its results with grid_dependency_wait(), so that its own launch costs no gap (~1 us of a 10 us call).  (Its input pointers carry no
-// __restrict__: a load through the non-coherent path may not start before the wait.)
-__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Every operator kernel is launched while its predecessor in the stream still runs (programmatic dependent launch) and begins with
+// grid_dependency(): it waits until that kernel has completed and its writes are visible, and then lets the next one be launched.  Wait
+// first, then release: at most two neighbouring kernels overlap, and nothing is read or written before everything earlier is done.  What
+// it saves is the launch latency and ramp of each call.  A predecessor that does not release early -- a framework's kernel, a copy -- is
+// simply waited for, and so is this kernel by such a successor.
+// The result is 0, but the compiler does not know that: added to the block index it makes every address depend on the wait, so that no
+// read-only load (__ldg, const __restrict__), which a memory clobber does not hold back, can be scheduled ahead of it.
+__device__ __forceinline__ uint32_t grid_dependency() {
+    uint32_t zero;
+    asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, 0;" : "=r"(zero)::"memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    return zero;
+}
+// (errors are left for check_launch())
 template <class... P, class... A>
-inline int launch_dependent(void (*kernel)(P...), unsigned grid, unsigned threads, cudaStream_t st, A... args) {
+inline void launch(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
-    if (e != cudaSuccess) {
-        g_last_cuda_error = (int)e;
-        return JF_ERR_LAUNCH;
-    }
-    return JF_OK;
+    (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 inline bool mult32(int64_t v) { return v > 0 && (v % 32) == 0; }

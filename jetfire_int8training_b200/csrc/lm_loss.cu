@@ -46,8 +46,7 @@ __device__ __forceinline__ void block_lse(float& m, float& s) {
 // per row: lse[row] = log sum exp(logits[row, :]);  loss[row] = lse - logits[row, target]   (0 for an ignored target < 0)
 __global__ void __launch_bounds__(LM_THREADS) lm_loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const int64_t* __restrict__ targets,
                                                                 int64_t V, float* __restrict__ lse, float* __restrict__ loss) {
-    const int64_t row = blockIdx.x;
-    grid_launch_dependents();      // the mean over the rows, where it follows
+    const int64_t row = blockIdx.x + grid_dependency();
     const __nv_bfloat16* x = logits + row * V;
     float m = -INFINITY, s = 0.f;
     const int64_t chunks = V / 8;
@@ -92,12 +91,13 @@ __global__ void __launch_bounds__(LM_THREADS) lm_loss_fwd_kernel(const __nv_bflo
 __global__ void __launch_bounds__(LM_THREADS) lm_loss_bwd_kernel(__nv_bfloat16* __restrict__ logits, const int64_t* __restrict__ targets,
                                                                 const float* __restrict__ lse, const float* __restrict__ grad_out,
                                                                 const float* __restrict__ count, float inv_count, int64_t V) {
-    const int64_t row = blockIdx.x;
+    const uint32_t zero = grid_dependency();
+    const int64_t row = blockIdx.x + zero;
     __nv_bfloat16* x = logits + row * V;
     const int64_t t = targets[row];
     const bool live = t >= 0 && t < V;
     // the mean's gradient: upstream / (number of counted positions), from device memory when the host does not know the number
-    const float scale = live ? (count ? __fdiv_rn(__ldg(grad_out), __ldg(count)) : __ldg(grad_out)) * inv_count : 0.f;
+    const float scale = live ? (count ? __fdiv_rn(__ldg(grad_out + zero), __ldg(count + zero)) : __ldg(grad_out + zero)) * inv_count : 0.f;
     const float l2 = lse[row] * 1.4426950408889634f;
     const int64_t chunks = V / 8;
     for (int64_t c = threadIdx.x; c < chunks; c += LM_THREADS) {
@@ -128,12 +128,12 @@ __global__ void __launch_bounds__(LM_THREADS) lm_loss_bwd_kernel(__nv_bfloat16* 
 // mean = sum(loss) / count, count = number of targets in [0, V), at least 1.  One CTA: a few thousand values.
 __global__ void __launch_bounds__(1024) lm_loss_mean_kernel(const float* loss, const int64_t* __restrict__ targets, int64_t rows, int64_t V, float* __restrict__ mean,
                                                             float* __restrict__ count) {
+    const uint32_t zero = grid_dependency();
     __shared__ float ssum[32];
     __shared__ int scnt[32];
-    grid_dependency_wait();
     float a = 0.f;
     int n = 0;
-    for (int64_t r = threadIdx.x; r < rows; r += 1024) {
+    for (int64_t r = threadIdx.x + zero; r < rows; r += 1024) {
         a += loss[r];
         const int64_t t = __ldg(targets + r);
         n += (t >= 0 && t < V) ? 1 : 0;
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(1024) lm_loss_mean_kernel(const float* loss, c
 // dst += src widened: the LM head's bf16 gradient joins the embedding's fp32 gradient of the same matrix.  10 bytes per element, eight
 // elements per thread (torch's type-promoting add took 127 us for 38.6 M elements, 3 TB/s).
 __global__ void __launch_bounds__(256) add_widened_kernel(float* __restrict__ dst, const __nv_bfloat16* __restrict__ src, int64_t n8) {
-    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    const int64_t i = (int64_t)(blockIdx.x + grid_dependency()) * 256 + threadIdx.x;
     if (i >= n8) return;
     float f[8];
     bf16x8_to_float(__ldg(reinterpret_cast<const uint4*>(src) + i), f);
@@ -175,7 +175,7 @@ int jf_add_widened(float* dst, const void* src_bf16, int64_t n, void* stream) {
     if (!dst || !src_bf16) return JF_ERR_NULL;
     if (n <= 0 || n % 8 != 0 || n / 2048 >= (int64_t(1) << 31)) return JF_ERR_SHAPE;
     if (!aligned16(dst) || !aligned16(src_bf16)) return JF_ERR_ALIGN;
-    add_widened_kernel<<<(unsigned)((n / 8 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(dst, (const __nv_bfloat16*)src_bf16, n / 8);
+    jf::launch(add_widened_kernel, (unsigned)((n / 8 + 255) / 256), 256, 0, (cudaStream_t)stream, dst, (const __nv_bfloat16*)src_bf16, n / 8);
     return check_launch();
 }
 
@@ -184,7 +184,7 @@ int jf_lm_loss_forward(const void* logits_bf16, const int64_t* targets, int64_t 
     if (!logits_bf16 || !targets || !lse || !loss_rows) return JF_ERR_NULL;
     if (rows <= 0 || V <= 0 || rows >= (int64_t(1) << 31)) return JF_ERR_SHAPE;
     if (!aligned16(logits_bf16) || (V % 8 != 0 && rows > 1)) return JF_ERR_ALIGN;     // every row must start on a 16-byte boundary
-    lm_loss_fwd_kernel<<<(unsigned)rows, LM_THREADS, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)logits_bf16, targets, V, lse, loss_rows);
+    jf::launch(lm_loss_fwd_kernel, (unsigned)rows, LM_THREADS, 0, (cudaStream_t)stream, (const __nv_bfloat16*)logits_bf16, targets, V, lse, loss_rows);
     return check_launch();
 }
 
@@ -192,7 +192,8 @@ int jf_lm_loss_forward_mean(const void* logits_bf16, const int64_t* targets, int
                             float* count, void* stream) {
     if (!mean || !count) return JF_ERR_NULL;
     if (int e = jf_lm_loss_forward(logits_bf16, targets, rows, V, lse, loss_rows, stream)) return e;
-    return launch_dependent(lm_loss_mean_kernel, 1, 1024, (cudaStream_t)stream, (const float*)loss_rows, targets, rows, V, mean, count);
+    jf::launch(lm_loss_mean_kernel, 1, 1024, 0, (cudaStream_t)stream, loss_rows, targets, rows, V, mean, count);
+    return check_launch();
 }
 
 static int lm_loss_backward(void* logits_bf16, const int64_t* targets, const float* lse, const float* grad_out, const float* count, float inv_count,
@@ -200,7 +201,7 @@ static int lm_loss_backward(void* logits_bf16, const int64_t* targets, const flo
     if (!logits_bf16 || !targets || !lse || !grad_out) return JF_ERR_NULL;
     if (rows <= 0 || V <= 0 || rows >= (int64_t(1) << 31)) return JF_ERR_SHAPE;
     if (!aligned16(logits_bf16) || (V % 8 != 0 && rows > 1)) return JF_ERR_ALIGN;
-    lm_loss_bwd_kernel<<<(unsigned)rows, LM_THREADS, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)logits_bf16, targets, lse, grad_out, count, inv_count, V);
+    jf::launch(lm_loss_bwd_kernel, (unsigned)rows, LM_THREADS, 0, (cudaStream_t)stream, (__nv_bfloat16*)logits_bf16, targets, lse, grad_out, count, inv_count, V);
     return check_launch();
 }
 

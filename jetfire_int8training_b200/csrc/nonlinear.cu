@@ -70,7 +70,7 @@ template <int TW, class Raw, bool PREFETCH, class LoadF, class ProcF>
 __device__ __forceinline__ void for_each_tile(int64_t M, int64_t N, LoadF&& load, ProcF&& proc) {
     const int64_t tiles_n = (N + TW - 1) / TW, total = (M / QB) * tiles_n;
     const int64_t stride = (int64_t)gridDim.x * WARPS;
-    int64_t tile = (int64_t)blockIdx.x * WARPS + (threadIdx.x >> 5);
+    int64_t tile = (int64_t)(blockIdx.x + grid_dependency()) * WARPS + (threadIdx.x >> 5);
     if (tile >= total) return;
     Tile t = make_tile<TW>(tile, tiles_n, N);
     Raw cur;
@@ -467,7 +467,8 @@ constexpr int DQ_THREADS = 128;
 
 __global__ void __launch_bounds__(DQ_THREADS)
 dequantize_kernel(const int8_t* __restrict__ q, const __half* __restrict__ s, int64_t M, int64_t N, float* __restrict__ y) {
-    const int64_t col = ((int64_t)blockIdx.x * DQ_THREADS + threadIdx.x) * 4;
+    const uint32_t block_x = blockIdx.x + grid_dependency();
+    const int64_t col = ((int64_t)block_x * DQ_THREADS + threadIdx.x) * 4;
     if (col >= N) return;
     const int64_t row0 = (int64_t)blockIdx.y * QB;
     const __half2 s2 = __half2half2(__ldg(s + blockIdx.y * (N / QB) + (col >> 5)));
@@ -501,8 +502,9 @@ constexpr int TR_TILE = 128;
 
 __global__ void __launch_bounds__(THREADS)
 transpose_kernel(const int8_t* __restrict__ x, int64_t M, int64_t N, int8_t* __restrict__ y) {
+    const uint32_t block_x = blockIdx.x + grid_dependency();
     __shared__ __align__(16) uint32_t tile[TR_TILE * TR_TILE / 4];
-    const int64_t R0 = (int64_t)blockIdx.y * TR_TILE, C0 = (int64_t)blockIdx.x * TR_TILE;
+    const int64_t R0 = (int64_t)blockIdx.y * TR_TILE, C0 = (int64_t)block_x * TR_TILE;
     const int t = threadIdx.x;
     {
         const int chunk = t & 7;
@@ -846,12 +848,12 @@ ln_bwd_kernel(const int8_t* __restrict__ qx, const __half* __restrict__ sx, cons
               const __half* __restrict__ sg, const float* __restrict__ gamma, const float* __restrict__ mean,
               const float* __restrict__ rstd, int64_t M, int64_t N, int8_t* __restrict__ qd, __half* __restrict__ sd,
               float* __restrict__ dw_partial, SrCfg sr) {
+    const uint32_t block_x = blockIdx.x + grid_dependency();
     constexpr int NP = Geo<TW>::NP, WPS = 128 / TW, PAIRS = WARPS / WPS;   // WPS warps per slab tile, PAIRS slab tiles per CTA
-    grid_launch_dependents();                          // the dgamma reduction
     __shared__ float2 row_part[PAIRS][WPS][QB];        // [slab tile][part][row of the tile] = (sum xhat*wdy, sum wdy) over the part
     const int warp = threadIdx.x >> 5, pair = warp / WPS, half = warp % WPS;
     const int64_t slabs_n = (N + 127) / 128, tiles_n_ = (N + TW - 1) / TW;
-    const int64_t slab_tile = (int64_t)blockIdx.x * PAIRS + pair;          // index of the 32 x 128 slab tile
+    const int64_t slab_tile = (int64_t)block_x * PAIRS + pair;          // index of the 32 x 128 slab tile
     if (slab_tile >= (M / QB) * slabs_n) return;                           // both warps of a pair leave together
     const int64_t tm_ = (int64_t)((uint32_t)slab_tile / (uint32_t)slabs_n);                      // 32-bit division
     const int64_t tn_ = (int64_t)((uint32_t)slab_tile % (uint32_t)slabs_n) * WPS + half;
@@ -960,10 +962,10 @@ ln_bwd_kernel(const int8_t* __restrict__ qx, const __half* __restrict__ sx, cons
 // dgamma[n] = sum over the M/32 partial rows: 8 interleaved row groups per column (thread (x, g) sums rows g, g+8, ...), then the
 // 8 group sums in ascending order -- a fixed order, so the result is deterministic.  Block = 32 columns x 8 groups.
 __global__ void __launch_bounds__(256) ln_bwd_dw_kernel(const float* partial, int64_t rows, int64_t N, float* __restrict__ dgamma) {
+    const uint32_t block_x = blockIdx.x + grid_dependency();
     __shared__ float red[8][32];
     const int tx = threadIdx.x & 31, g = threadIdx.x >> 5;
-    const int64_t n = (int64_t)blockIdx.x * 32 + tx;
-    grid_dependency_wait();
+    const int64_t n = (int64_t)block_x * 32 + tx;
     float a = 0.f;
     if (n < N) {
         int64_t r = g;
@@ -1050,10 +1052,11 @@ __device__ __forceinline__ void emit_block4(RowF&& rowf /* i -> the lane's float
 template <typename T, bool SR>
 __global__ void __launch_bounds__(THREADS, 3)
 quantize4_kernel(const T* __restrict__ x, int64_t M, int64_t N, int8_t* __restrict__ q, __half* __restrict__ s, SrCfg sr) {
+    const uint32_t block_x = blockIdx.x + grid_dependency();
     const int64_t blocks_n = N / QB, total = (M / QB) * blocks_n;
     const int64_t stride = (int64_t)gridDim.x * WARPS;
     const int lane = threadIdx.x & 31, r = lane >> 3, c = lane & 7;
-    int64_t blk = (int64_t)blockIdx.x * WARPS + (threadIdx.x >> 5);
+    int64_t blk = (int64_t)block_x * WARPS + (threadIdx.x >> 5);
     if (blk >= total) return;
     auto base_of = [&](int64_t b) {
         const int64_t tm = (int64_t)((uint32_t)b / (uint32_t)blocks_n), tn = (int64_t)((uint32_t)b % (uint32_t)blocks_n);
@@ -1112,12 +1115,13 @@ struct QuantizeJobs {
 
 template <typename T>
 __global__ void __launch_bounds__(THREADS, 3) quantize_multi_kernel(const QuantizeJobs jobs) {
+    const uint32_t block_x = blockIdx.x + grid_dependency();
     const int64_t total = jobs.first_block[jobs.count];
     const int64_t stride = (int64_t)gridDim.x * WARPS;
     const int lane = threadIdx.x & 31, r = lane >> 3, c = lane & 7;
     using Raw = typename std::conditional<sizeof(T) == 4, float4, uint2>::type;
     SrCfg sr{};
-    for (int64_t g = (int64_t)blockIdx.x * WARPS + (threadIdx.x >> 5); g < total; g += stride) {
+    for (int64_t g = (int64_t)block_x * WARPS + (threadIdx.x >> 5); g < total; g += stride) {
         int j = 0;
 #pragma unroll
         for (int k = 1; k < QMULTI_MAX; ++k) j += (k < jobs.count && g >= jobs.first_block[k]) ? 1 : 0;
@@ -1183,14 +1187,14 @@ __global__ void __launch_bounds__(THREADS, 3)
 add_kernel(const T* __restrict__ x1, const int8_t* __restrict__ q2, const __half* __restrict__ s2, int64_t M, int64_t N,
            OutT* __restrict__ y1, int8_t* __restrict__ qy, __half* __restrict__ sy, float* __restrict__ part_sum,
            float* __restrict__ part_sq, SrCfg sr) {
+    const uint32_t block_x = blockIdx.x + grid_dependency();
     // Row statistics: the four warps of a 128-column slab leave each lane's sums (of its four columns of a row) in shared memory.  They are
     // added per lane in column order and then over the eight lanes as a tree -- the order of one warp that walks the four blocks, so that
     // mean and rstd, which decide roundings of everything behind them, do not depend on how the work is split.
     __shared__ float row_sum[MEANVAR ? WARPS : 1][MEANVAR ? 256 : 1], row_sq[MEANVAR ? WARPS : 1][MEANVAR ? 256 : 1];   // [warp][8 row + lane]
-    if (MEANVAR) grid_launch_dependents();                    // the statistics' last step
     const int64_t blocks_n = N / QB;                          // blocks per row of blocks
     const int64_t slabs_n = (blocks_n + 3) / 4;               // MEANVAR: warps are numbered by slab, a short last slab leaves some idle
-    const int64_t item = (int64_t)blockIdx.x * WARPS + (threadIdx.x >> 5);
+    const int64_t item = (int64_t)block_x * WARPS + (threadIdx.x >> 5);
     const int64_t per_row = MEANVAR ? 4 * slabs_n : blocks_n;
     const bool inside = item < (M / QB) * per_row;
     const int64_t tm = (int64_t)((uint32_t)item / (uint32_t)per_row), tn = (int64_t)((uint32_t)item % (uint32_t)per_row);   // 32-bit division
@@ -1234,7 +1238,7 @@ add_kernel(const T* __restrict__ x1, const int8_t* __restrict__ q2, const __half
         const int k = threadIdx.x, row = k >> 3;                       // thread = (row of the slab, lane of the row)
 #pragma unroll
         for (int slab = 0; slab < WARPS / 4; ++slab) {                 // the CTA's two slabs
-            const int64_t first = (int64_t)blockIdx.x * WARPS + 4 * slab;
+            const int64_t first = (int64_t)block_x * WARPS + 4 * slab;
             float a = row_sum[4 * slab][k], b = row_sq[4 * slab][k];
 #pragma unroll
             for (int w = 1; w < 4; ++w) { a = __fadd_rn(a, row_sum[4 * slab + w][k]); b = __fadd_rn(b, row_sq[4 * slab + w][k]); }
@@ -1255,8 +1259,8 @@ add_kernel(const T* __restrict__ x1, const int8_t* __restrict__ q2, const __half
 // mean = sum/N; rstd = 1/sqrt(sumsq/N - mean^2)
 __global__ void meanvar_finish_kernel(const float* part_sum, const float* part_sq, int64_t M, int64_t tiles_n,
                                       int64_t N, float* __restrict__ mean, float* __restrict__ rstd) {
-    const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    grid_dependency_wait();
+    const uint32_t block_x = blockIdx.x + grid_dependency();
+    const int64_t row = (int64_t)block_x * blockDim.x + threadIdx.x;
     if (row >= M) return;
     float a = 0.f, b = 0.f;
     for (int64_t k = 0; k < tiles_n; ++k) {
@@ -1311,14 +1315,14 @@ static void launch_quantize(const void* x, int64_t M, int64_t N, int8_t* q, __ha
     const T* xp = (const T*)x;
     if (qt) {
         const unsigned grid = grid_for<64>(M, N, persistent_ctas(2));
-        if (stochastic) quantize_kernel<T, 64, true, true><<<grid, THREADS, 0, st>>>(xp, M, N, q, s, qt, sr);
-        else quantize_kernel<T, 64, false, true><<<grid, THREADS, 0, st>>>(xp, M, N, q, s, qt, sr);
+        if (stochastic) jf::launch(quantize_kernel<T, 64, true, true>, grid, THREADS, 0, st, xp, M, N, q, s, qt, sr);
+        else jf::launch(quantize_kernel<T, 64, false, true>, grid, THREADS, 0, st, xp, M, N, q, s, qt, sr);
     } else {
         const unsigned grid = grid_for<32>(M, N, persistent_ctas(3));
         // round-to-nearest: the 4-columns-per-lane mapping (whole sectors per access); stochastic rounding: the 16-columns-per-lane
         // mapping, where a lane owns whole 8-element Philox groups (measured on [8192 x 3072] bf16: 31.1 us against 33.4 us)
-        if (stochastic) quantize_kernel<T, 32, true, false><<<grid, THREADS, 0, st>>>(xp, M, N, q, s, nullptr, sr);
-        else quantize4_kernel<T, false><<<grid, THREADS, 0, st>>>(xp, M, N, q, s, sr);
+        if (stochastic) jf::launch(quantize_kernel<T, 32, true, false>, grid, THREADS, 0, st, xp, M, N, q, s, nullptr, sr);
+        else jf::launch(quantize4_kernel<T, false>, grid, THREADS, 0, st, xp, M, N, q, s, sr);
     }
 }
 
@@ -1367,9 +1371,9 @@ static void launch_add(const void* x1, const int8_t* q2, const __half* s2, int64
     OutT* yp = (OutT*)y1;
     const int64_t blocks = (M / QB) * (N / QB), padded = (M / QB) * 4 * ((N + 127) / 128);
     const unsigned grid_b = (unsigned)((blocks + WARPS - 1) / WARPS), grid_s = (unsigned)((padded + WARPS - 1) / WARPS);
-    if (meanvar) add_kernel<T, OutT, true, false><<<grid_s, THREADS, 0, st>>>(xp, q2, s2, M, N, yp, qy, sy, ps, pq, sr);
-    else if (stochastic) add_kernel<T, OutT, false, true><<<grid_b, THREADS, 0, st>>>(xp, q2, s2, M, N, yp, qy, sy, ps, pq, sr);
-    else add_kernel<T, OutT, false, false><<<grid_b, THREADS, 0, st>>>(xp, q2, s2, M, N, yp, qy, sy, ps, pq, sr);
+    if (meanvar) jf::launch(add_kernel<T, OutT, true, false>, grid_s, THREADS, 0, st, xp, q2, s2, M, N, yp, qy, sy, ps, pq, sr);
+    else if (stochastic) jf::launch(add_kernel<T, OutT, false, true>, grid_b, THREADS, 0, st, xp, q2, s2, M, N, yp, qy, sy, ps, pq, sr);
+    else jf::launch(add_kernel<T, OutT, false, false>, grid_b, THREADS, 0, st, xp, q2, s2, M, N, yp, qy, sy, ps, pq, sr);
 }
 
 extern "C" {
@@ -1426,8 +1430,8 @@ int jf_int8_quantize_parts(int count, const void* const* x, int x_dtype, int64_t
         for (int k = 0; k < count; ++k) p.p[k] = (const T*)x[k];
         p.cols = cols;
         const unsigned grid = grid_for<32>(M, N, persistent_ctas(3));
-        if (stochastic) quantize_kernel<T, 32, true, false, Parts<T>><<<grid, THREADS, 0, (cudaStream_t)stream>>>(p, M, N, q, (__half*)s, nullptr, sr);
-        else quantize_kernel<T, 32, false, false, Parts<T>><<<grid, THREADS, 0, (cudaStream_t)stream>>>(p, M, N, q, (__half*)s, nullptr, sr);
+        if (stochastic) jf::launch(quantize_kernel<T, 32, true, false, Parts<T>>, grid, THREADS, 0, (cudaStream_t)stream, p, M, N, q, (__half*)s, nullptr, sr);
+        else jf::launch(quantize_kernel<T, 32, false, false, Parts<T>>, grid, THREADS, 0, (cudaStream_t)stream, p, M, N, q, (__half*)s, nullptr, sr);
     };
     switch (x_dtype) {
         case JF_F32: launch(float()); break;
@@ -1460,9 +1464,9 @@ int jf_int8_quantize_multi(int count, const void* const* x, int x_dtype, const i
     const unsigned grid = (unsigned)(ctas > cap ? cap : ctas);
     cudaStream_t st = (cudaStream_t)stream;
     switch (x_dtype) {
-        case JF_F32: quantize_multi_kernel<float><<<grid, THREADS, 0, st>>>(jobs); break;
-        case JF_F16: quantize_multi_kernel<__half><<<grid, THREADS, 0, st>>>(jobs); break;
-        case JF_BF16: quantize_multi_kernel<__nv_bfloat16><<<grid, THREADS, 0, st>>>(jobs); break;
+        case JF_F32: jf::launch(quantize_multi_kernel<float>, grid, THREADS, 0, st, jobs); break;
+        case JF_F16: jf::launch(quantize_multi_kernel<__half>, grid, THREADS, 0, st, jobs); break;
+        case JF_BF16: jf::launch(quantize_multi_kernel<__nv_bfloat16>, grid, THREADS, 0, st, jobs); break;
         default: return JF_ERR_DTYPE;
     }
     return check_launch();
@@ -1475,7 +1479,7 @@ int jf_int8_dequantize(const int8_t* q, const void* s, int64_t M, int64_t N, flo
     cudaStream_t st = (cudaStream_t)stream;
     if (M / QB > 65535) return JF_ERR_SHAPE;     // one grid row per row of blocks
     const dim3 grid((unsigned)((N / 4 + DQ_THREADS - 1) / DQ_THREADS), (unsigned)(M / QB));
-    dequantize_kernel<<<grid, DQ_THREADS, 0, st>>>(q, (const __half*)s, M, N, y);
+    jf::launch(dequantize_kernel, grid, DQ_THREADS, 0, st, q, (const __half*)s, M, N, y);
     return check_launch();
 }
 
@@ -1486,7 +1490,7 @@ int jf_int8_transpose(const int8_t* x, int64_t M, int64_t N, int8_t* y, void* st
     cudaStream_t st = (cudaStream_t)stream;
     if ((M + TR_TILE - 1) / TR_TILE > 65535) return JF_ERR_SHAPE;     // one grid row per 128 rows
     const dim3 grid((unsigned)((N + TR_TILE - 1) / TR_TILE), (unsigned)((M + TR_TILE - 1) / TR_TILE));
-    transpose_kernel<<<grid, THREADS, 0, st>>>(x, M, N, y);
+    jf::launch(transpose_kernel, grid, THREADS, 0, st, x, M, N, y);
     return check_launch();
 }
 
@@ -1496,7 +1500,7 @@ int jf_int8_gelu_forward(const int8_t* qx, const void* sx, int64_t M, int64_t N,
     JF_REQUIRE_ALIGNED(qx); JF_REQUIRE_ALIGNED(qy);
     cudaStream_t st = (cudaStream_t)stream;
     if (int e = ensure_gelu_table(st, false)) return e;
-    gelu_fwd_kernel<<<grid_for<32>(M, N, persistent_ctas(4)), THREADS, 0, st>>>(qx, (const __half*)sx, M, N, qy, (__half*)sy);
+    jf::launch(gelu_fwd_kernel, grid_for<32>(M, N, persistent_ctas(4)), THREADS, 0, st, qx, (const __half*)sx, M, N, qy, (__half*)sy);
     return check_launch();
 }
 
@@ -1511,8 +1515,8 @@ int jf_int8_gelu_backward(const int8_t* qx, const void* sx, const int8_t* qg, co
     const __half* sxh = (const __half*)sx; const __half* sgh = (const __half*)sg; __half* sdh = (__half*)sd;
     if (int e = ensure_gelu_table(st, true)) return e;
     const unsigned grid = grid_for<32>(M, N, persistent_ctas(3));
-    if (stochastic) gelu_bwd_kernel<true><<<grid, THREADS, 0, st>>>(qx, sxh, qg, sgh, M, N, qd, sdh, sr);
-    else gelu_bwd_kernel<false><<<grid, THREADS, 0, st>>>(qx, sxh, qg, sgh, M, N, qd, sdh, sr);
+    if (stochastic) jf::launch(gelu_bwd_kernel<true>, grid, THREADS, 0, st, qx, sxh, qg, sgh, M, N, qd, sdh, sr);
+    else jf::launch(gelu_bwd_kernel<false>, grid, THREADS, 0, st, qx, sxh, qg, sgh, M, N, qd, sdh, sr);
     return check_launch();
 }
 
@@ -1523,7 +1527,7 @@ int jf_int8_layernorm_forward(const int8_t* qx, const void* sx, const float* gam
     if (int e = check_mn(M, N)) return e;
     JF_REQUIRE_ALIGNED(qx); JF_REQUIRE_ALIGNED(qy); JF_REQUIRE_ALIGNED(gamma);
     cudaStream_t st = (cudaStream_t)stream;
-    ln_fwd_kernel<32><<<grid_for<32>(M, N, persistent_ctas(4)), THREADS, 0, st>>>(qx, (const __half*)sx, gamma, mean, rstd, M, N, qy, (__half*)sy);
+    jf::launch(ln_fwd_kernel<32>, grid_for<32>(M, N, persistent_ctas(4)), THREADS, 0, st, qx, (const __half*)sx, gamma, mean, rstd, M, N, qy, (__half*)sy);
     return check_launch();
 }
 
@@ -1543,10 +1547,11 @@ int jf_int8_layernorm_backward(const int8_t* qx, const void* sx, const int8_t* q
     const int64_t slab_tiles = (M / QB) * ((N + 127) / 128);
     const unsigned grid = (unsigned)((slab_tiles + WARPS / 2 - 1) / (WARPS / 2));   // two warps per 32 x 128 slab tile
     const __half* sxh = (const __half*)sx; const __half* sgh = (const __half*)sg; __half* sdh = (__half*)sd;
-    if (stochastic) ln_bwd_kernel<true><<<grid, THREADS, 0, st>>>(qx, sxh, qg, sgh, gamma, mean, rstd, M, N, qd, sdh, scratch, sr);
-    else ln_bwd_kernel<false><<<grid, THREADS, 0, st>>>(qx, sxh, qg, sgh, gamma, mean, rstd, M, N, qd, sdh, scratch, sr);
+    if (stochastic) jf::launch(ln_bwd_kernel<true>, grid, THREADS, 0, st, qx, sxh, qg, sgh, gamma, mean, rstd, M, N, qd, sdh, scratch, sr);
+    else jf::launch(ln_bwd_kernel<false>, grid, THREADS, 0, st, qx, sxh, qg, sgh, gamma, mean, rstd, M, N, qd, sdh, scratch, sr);
     if (int e = check_launch()) return e;
-    return launch_dependent(ln_bwd_dw_kernel, (unsigned)((N + 31) / 32), 256, st, (const float*)scratch, M / QB, N, dgamma);
+    jf::launch(ln_bwd_dw_kernel, (unsigned)((N + 31) / 32), 256, 0, st, scratch, M / QB, N, dgamma);
+    return check_launch();
 }
 
 static int add_impl(const void* x1, int x1_dtype, const int8_t* q2, const void* s2, int64_t M, int64_t N, void* y1, int y1_dtype, int8_t* qy,
@@ -1579,7 +1584,8 @@ static int add_impl(const void* x1, int x1_dtype, const int8_t* q2, const void* 
     }
     if (int e = check_launch()) return e;
     if (meanvar) {
-        return launch_dependent(meanvar_finish_kernel, (unsigned)((M + 63) / 64), 64, st, (const float*)ps, (const float*)pq, M, tiles_n, N, mean, rstd);
+        jf::launch(meanvar_finish_kernel, (unsigned)((M + 63) / 64), 64, 0, st, ps, pq, M, tiles_n, N, mean, rstd);
+        return check_launch();
     }
     return JF_OK;
 }
