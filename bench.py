@@ -190,8 +190,8 @@ def run_ours(args):
         return (torch.rand(r, c, generator=g, device=dev) * 0.099 + 1e-3).half()
     SX, SW, SG = scales(M // 32, K // 32), scales(N // 32, K // 32), scales(M // 32, N // 32)
 
-    # forward, dgrad, wgrad (+ the split-K reduction)
-    launches_per_step = 3 + (1 if L.jf_igemm_wgrad_plan(N, K, M, 0) > 1 else 0)
+    # forward, both gradients (+ the split-K reduction)
+    launches_per_step = 1 + L.jf_igemm_backward_launches(M, N, K, 0)
     fwd_ev = []
     # data-parallel exchange: the mean of dW over the ranks, one NCCL all-reduce (AVG) per step behind the weight-gradient GEMM
     reducer = MeanReducer(device=dev)

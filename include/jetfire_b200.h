@@ -188,6 +188,18 @@ int jf_igemm_wgrad(const int8_t* g, int g_transposed, const int8_t* x, const voi
                    int64_t sg_stride_m, const void* sx, int64_t sx_stride_k, int64_t sx_stride_n, int64_t M, int64_t N,
                    int64_t K, int out_dtype, void* dw, int split_k, float* scratch, void* op16, int64_t op16_bytes, void* stream);
 
+/* Both gradients of a linear layer (plus the split-K sum, when there is one): dX = dY W as jf_igemm_dgrad and dW = dY^T X as
+ * jf_igemm_wgrad with g_transposed = 0, bit for bit.  g int8 [tokens, cout], w int8 [cout, cin], x int8 [tokens, cin], all row-major;
+ * scale strides in block rows and block columns of each.  Where that is faster, one launch in which the tiles of both products share the
+ * SMs, so that neither leaves a last round of them partly idle; jf_igemm_backward_launches gives the number of kernels (1 to 3). */
+int jf_igemm_backward(const int8_t* g, const int8_t* w, const int8_t* x, const void* sg, int64_t sg_stride_m, int64_t sg_stride_n,
+                      const void* sw, int64_t sw_stride_n, int64_t sw_stride_k, const void* sx, int64_t sx_stride_m,
+                      int64_t sx_stride_k, int64_t tokens, int64_t cout, int64_t cin, int out_mode, int8_t* dx8, void* sdx,
+                      void* dx16, int stochastic, const float* noise, uint64_t seed, uint64_t offset, int dw_dtype, void* dw,
+                      int split_k, float* scratch, void* stream);
+
+int jf_igemm_backward_launches(int64_t tokens, int64_t cout, int64_t cin, int split_k);
+
 /* Effective split-K the library would use for (M,N,K,split_k) on the current device (>= 1), so that the caller can
  * size `scratch`.  Host-only; launches nothing. */
 int jf_igemm_wgrad_plan(int64_t M, int64_t N, int64_t K, int split_k);

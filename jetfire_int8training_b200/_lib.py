@@ -36,6 +36,9 @@ SIGNATURES = {
                         _u64, _u64, _vp, _i64, _vp], _int),
     "jf_igemm_wgrad": ([_vp, _int, _vp, _vp, _i64, _i64, _vp, _i64, _i64, _i64, _i64, _i64, _int, _vp, _int, _vp, _vp, _i64,
                         _vp], _int),
+    "jf_igemm_backward": ([_vp, _vp, _vp, _vp, _i64, _i64, _vp, _i64, _i64, _vp, _i64, _i64, _i64, _i64, _i64, _int, _vp, _vp, _vp, _int, _vp,
+                           _u64, _u64, _int, _vp, _int, _vp, _vp], _int),
+    "jf_igemm_backward_launches": ([_i64, _i64, _i64, _int], _int),
     "jf_igemm_wgrad_plan": ([_i64, _i64, _i64, _int], _int),
     "jf_igemm_int32": ([_vp, _vp, _i64, _i64, _i64, _vp, _vp], _int),
     "jf_igemm_error_flag": ([], _int),

@@ -18,6 +18,7 @@
 // leaves its loops, waits (bounded) for its copies and MMAs in flight and frees its tensor memory.
 #include <cuda.h>
 
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -56,6 +57,10 @@ struct GemmParams {
     int mode;
     int8_t* out8; __half* out_scale; __half* out16; float* out32; int32_t* out_i32;
     int stochastic; const float* noise; uint64_t offset; PhiloxKeys keys;
+};
+struct GemmPair {                       // the parameters of PairWalk
+    GemmParams g[2];                    // dX, dW
+    uint32_t long_one, rounds, short_from, level, short_items;
 };
 
 __device__ int g_gemm_error = 0;   // 0 = ok; otherwise the code of the first wait that expired
@@ -96,13 +101,15 @@ __device__ __forceinline__ void scale_accumulate(uint64_t (&acc2)[16], const uin
 }
 
 // Re-quantise / convert one 32x32 block held as 32 lanes x 16 packed pairs and store it.  Two values per instruction throughout.
+enum StoreKind : int { STORE_DENSE = 1, STORE_QUANTISED = 2 };
+template <int KINDS>
 __device__ __forceinline__ void store_block(const GemmParams& p, const uint64_t (&acc2)[16], int64_t row, int64_t col, int64_t rowblk,
                                             int64_t colblk, int64_t split, int lane) {
-    if (p.mode == MODE_INT32) {
+    if ((KINDS & STORE_DENSE) && p.mode == MODE_INT32) {
         int4* dst = reinterpret_cast<int4*>(p.out_i32 + row * p.N + col);
 #pragma unroll
         for (int k = 0; k < 8; ++k) dst[k] = make_int4((int)acc2[2 * k], (int)(acc2[2 * k] >> 32), (int)acc2[2 * k + 1], (int)(acc2[2 * k + 1] >> 32));
-    } else if (p.mode == MODE_F32) {
+    } else if ((KINDS & STORE_DENSE) && p.mode == MODE_F32) {
         float4* dst = reinterpret_cast<float4*>(p.out32 + (split * p.M + row) * p.N + col);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
@@ -111,7 +118,7 @@ __device__ __forceinline__ void store_block(const GemmParams& p, const uint64_t 
             f2_unpack(acc2[2 * k + 1], v.z, v.w);
             dst[k] = v;
         }
-    } else if (p.mode == MODE_F16) {
+    } else if ((KINDS & STORE_DENSE) && p.mode == MODE_F16) {
         int4* dst = reinterpret_cast<int4*>(p.out16 + row * p.N + col);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -124,7 +131,7 @@ __device__ __forceinline__ void store_block(const GemmParams& p, const uint64_t 
             }
             dst[k] = *reinterpret_cast<int4*>(h);
         }
-    } else {
+    } else if (KINDS & STORE_QUANTISED) {
         float m = 0.f;
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
@@ -330,6 +337,62 @@ static inline int check_gemm_dims(int64_t M, int64_t N, int64_t K) {
     return JF_OK;
 }
 
+// What the entry points of the two gradients check and fill in.
+static int dgrad_params(GemmParams& p, const int8_t* g, const int8_t* w, const void* sg, int64_t sg_stride_m, int64_t sg_stride_k,
+                        const void* sw, int64_t sw_stride_k, int64_t sw_stride_n, int64_t M, int64_t N, int64_t K, int out_mode, int8_t* dx8,
+                        void* sdx, void* dx16, int stochastic, const float* noise, uint64_t seed, uint64_t offset) {
+    if (!g || !w || !sg || !sw) return JF_ERR_NULL;
+    if (int e = check_gemm_dims(M, N, K)) return e;
+    if (!aligned16(g) || !aligned16(w) || (noise && !aligned16(noise))) return JF_ERR_ALIGN;
+    p.M = M; p.N = N; p.K = K; p.splits = 1; p.kb_per_split = K / QB;
+    p.sa = (const __half*)sg; p.sa_sm = sg_stride_m; p.sa_sk = sg_stride_k;
+    p.sb = (const __half*)sw; p.sb_sn = sw_stride_n; p.sb_sk = sw_stride_k;
+    p.stochastic = stochastic; p.noise = noise; p.keys = make_philox_keys(seed, offset); p.offset = offset;
+    if (out_mode == JF_OUT_INT8) {
+        if (!dx8 || !sdx) return JF_ERR_NULL;
+        if (!aligned16(dx8)) return JF_ERR_ALIGN;
+        p.mode = MODE_INT8; p.out8 = dx8; p.out_scale = (__half*)sdx;
+    } else if (out_mode == JF_OUT_DEQUANT_F16) {
+        if (!dx16) return JF_ERR_NULL;
+        if (!aligned16(dx16)) return JF_ERR_ALIGN;
+        p.mode = MODE_DEQ16; p.out16 = (__half*)dx16;
+    } else {
+        return JF_ERR_ARG;
+    }
+    return JF_OK;
+}
+static int wgrad_params(GemmParams& p, const int8_t* g, const int8_t* x, const void* sg, int64_t sg_stride_k, int64_t sg_stride_m,
+                        const void* sx, int64_t sx_stride_k, int64_t sx_stride_n, int64_t M, int64_t N, int64_t K, int out_dtype, void* dw,
+                        int split_k, float* scratch) {
+    if (!g || !x || !sg || !sx || !dw) return JF_ERR_NULL;
+    if (int e = check_gemm_dims(M, N, K)) return e;
+    if (!aligned16(g) || !aligned16(x) || !aligned16(dw)) return JF_ERR_ALIGN;
+    if (out_dtype != JF_F16 && out_dtype != JF_F32) return JF_ERR_DTYPE;
+    DeviceInfo* di = nullptr;
+    if (int e = device_info(&di)) return e;
+    p.M = M; p.N = N; p.K = K;
+    p.splits = plan_splits(M, N, K, split_k, di->sm_count, &p.kb_per_split);
+    p.sa = (const __half*)sg; p.sa_sm = sg_stride_m; p.sa_sk = sg_stride_k;
+    p.sb = (const __half*)sx; p.sb_sn = sx_stride_n; p.sb_sk = sx_stride_k;
+    if (p.splits == 1) {
+        if (out_dtype == JF_F16) { p.mode = MODE_F16; p.out16 = (__half*)dw; }
+        else { p.mode = MODE_F32; p.out32 = (float*)dw; }
+        return JF_OK;
+    }
+    if (!scratch) return JF_ERR_NULL;
+    if (!aligned16(scratch)) return JF_ERR_ALIGN;
+    p.mode = MODE_F32; p.out32 = scratch;
+    return JF_OK;
+}
+static int reduce_splits(const GemmParams& p, const float* scratch, int out_dtype, void* dw, cudaStream_t st) {
+    if (p.splits == 1) return JF_OK;
+    const int64_t count = p.M * p.N;
+    const unsigned grid = (unsigned)((count / 4 + 255) / 256);
+    if (out_dtype == JF_F16) jf::launch(splitk_reduce_kernel<__half>, grid, 256, 0, st, scratch, p.splits, count, (__half*)dw);
+    else jf::launch(splitk_reduce_kernel<float>, grid, 256, 0, st, scratch, p.splits, count, (float*)dw);
+    return check_launch();
+}
+
 extern "C" {
 
 int jf_igemm_forward(const int8_t* x, const int8_t* w, const void* sx, int64_t sx_stride_m, int64_t sx_stride_k, const void* sw,
@@ -365,25 +428,9 @@ int jf_igemm_dgrad(const int8_t* g, const int8_t* w, const void* sg, int64_t sg_
                    int64_t sw_stride_k, int64_t sw_stride_n, int64_t M, int64_t N, int64_t K, int out_mode, int8_t* dx8, void* sdx,
                    void* dx16, int stochastic, const float* noise, uint64_t seed, uint64_t offset, void* op16, int64_t op16_bytes,
                    void* stream) {
-    if (!g || !w || !sg || !sw) return JF_ERR_NULL;
-    if (int e = check_gemm_dims(M, N, K)) return e;
-    if (!aligned16(g) || !aligned16(w) || (noise && !aligned16(noise))) return JF_ERR_ALIGN;
     GemmParams p{};
-    p.M = M; p.N = N; p.K = K; p.splits = 1; p.kb_per_split = K / QB;
-    p.sa = (const __half*)sg; p.sa_sm = sg_stride_m; p.sa_sk = sg_stride_k;
-    p.sb = (const __half*)sw; p.sb_sn = sw_stride_n; p.sb_sk = sw_stride_k;
-    p.stochastic = stochastic; p.noise = noise; p.keys = make_philox_keys(seed, offset); p.offset = offset;
-    if (out_mode == JF_OUT_INT8) {
-        if (!dx8 || !sdx) return JF_ERR_NULL;
-        if (!aligned16(dx8)) return JF_ERR_ALIGN;
-        p.mode = MODE_INT8; p.out8 = dx8; p.out_scale = (__half*)sdx;
-    } else if (out_mode == JF_OUT_DEQUANT_F16) {
-        if (!dx16) return JF_ERR_NULL;
-        if (!aligned16(dx16)) return JF_ERR_ALIGN;
-        p.mode = MODE_DEQ16; p.out16 = (__half*)dx16;
-    } else {
-        return JF_ERR_ARG;
-    }
+    if (int e = dgrad_params(p, g, w, sg, sg_stride_m, sg_stride_k, sw, sw_stride_k, sw_stride_n, M, N, K, out_mode, dx8, sdx, dx16,
+                             stochastic, noise, seed, offset)) return e;
     (void)op16; (void)op16_bytes;
     return launch_dgrad_layout(g, w, p, (cudaStream_t)stream);
 }
@@ -399,35 +446,41 @@ int jf_igemm_wgrad_plan(int64_t M, int64_t N, int64_t K, int split_k) {
 int jf_igemm_wgrad(const int8_t* g, int g_transposed, const int8_t* x, const void* sg, int64_t sg_stride_k, int64_t sg_stride_m,
                    const void* sx, int64_t sx_stride_k, int64_t sx_stride_n, int64_t M, int64_t N, int64_t K, int out_dtype, void* dw,
                    int split_k, float* scratch, void* op16, int64_t op16_bytes, void* stream) {
-    if (!g || !x || !sg || !sx || !dw) return JF_ERR_NULL;
-    if (int e = check_gemm_dims(M, N, K)) return e;
-    if (!aligned16(g) || !aligned16(x) || !aligned16(dw)) return JF_ERR_ALIGN;
-    if (out_dtype != JF_F16 && out_dtype != JF_F32) return JF_ERR_DTYPE;
-    DeviceInfo* di = nullptr;
-    if (int e = device_info(&di)) return e;
-    int64_t per = 0;
-    const int splits = plan_splits(M, N, K, split_k, di->sm_count, &per);
     GemmParams p{};
-    p.M = M; p.N = N; p.K = K; p.splits = splits; p.kb_per_split = per;
-    p.sa = (const __half*)sg; p.sa_sm = sg_stride_m; p.sa_sk = sg_stride_k;
-    p.sb = (const __half*)sx; p.sb_sn = sx_stride_n; p.sb_sk = sx_stride_k;
+    if (int e = wgrad_params(p, g, x, sg, sg_stride_k, sg_stride_m, sx, sx_stride_k, sx_stride_n, M, N, K, out_dtype, dw, split_k, scratch)) return e;
     cudaStream_t st = (cudaStream_t)stream;
     (void)op16; (void)op16_bytes;
-    auto launch = [&]() { return g_transposed ? launch_dgrad_layout(g, x, p, st) : launch_wgrad_layout(g, x, p, st); };
-    if (splits == 1) {
-        if (out_dtype == JF_F16) { p.mode = MODE_F16; p.out16 = (__half*)dw; }
-        else { p.mode = MODE_F32; p.out32 = (float*)dw; }
-        return launch();
-    }
-    if (!scratch) return JF_ERR_NULL;
-    if (!aligned16(scratch)) return JF_ERR_ALIGN;
-    p.mode = MODE_F32; p.out32 = scratch;
-    if (int e = launch()) return e;
-    const int64_t count = M * N;
-    const unsigned grid = (unsigned)((count / 4 + 255) / 256);
-    if (out_dtype == JF_F16) jf::launch(splitk_reduce_kernel<__half>, grid, 256, 0, st, scratch, splits, count, (__half*)dw);
-    else jf::launch(splitk_reduce_kernel<float>, grid, 256, 0, st, scratch, splits, count, (float*)dw);
-    return check_launch();
+    if (int e = g_transposed ? launch_dgrad_layout(g, x, p, st) : launch_wgrad_layout(g, x, p, st)) return e;
+    return reduce_splits(p, scratch, out_dtype, dw, st);
+}
+
+int jf_igemm_backward(const int8_t* g, const int8_t* w, const int8_t* x, const void* sg, int64_t sg_stride_m, int64_t sg_stride_n,
+                      const void* sw, int64_t sw_stride_n, int64_t sw_stride_k, const void* sx, int64_t sx_stride_m, int64_t sx_stride_k,
+                      int64_t tokens, int64_t cout, int64_t cin, int out_mode, int8_t* dx8, void* sdx, void* dx16, int stochastic,
+                      const float* noise, uint64_t seed, uint64_t offset, int dw_dtype, void* dw, int split_k, float* scratch, void* stream) {
+    GemmParams d{}, q{};
+    if (int e = dgrad_params(d, g, w, sg, sg_stride_m, sg_stride_n, sw, sw_stride_n, sw_stride_k, tokens, cin, cout, out_mode, dx8, sdx, dx16,
+                             stochastic, noise, seed, offset)) return e;
+    if (int e = wgrad_params(q, g, x, sg, sg_stride_m, sg_stride_n, sx, sx_stride_m, sx_stride_k, cout, cin, tokens, dw_dtype, dw, split_k,
+                             scratch)) return e;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (int e = launch_pair(g, w, x, d, q, st)) return e;
+    return reduce_splits(q, scratch, dw_dtype, dw, st);
+}
+
+int jf_igemm_backward_launches(int64_t tokens, int64_t cout, int64_t cin, int split_k) {
+    if (check_gemm_dims(tokens, cout, cin)) return JF_ERR_SHAPE;
+    int sm = 148;
+    DeviceInfo* di = nullptr;
+    if (device_info(&di) == JF_OK) sm = di->sm_count;
+    GemmPair pair{};
+    GemmParams &d = pair.g[0], &w = pair.g[1];
+    d.M = tokens; d.N = cin; d.K = cout; d.splits = 1; d.kb_per_split = cout / QB;
+    w.M = cout; w.N = cin; w.K = tokens; w.splits = plan_splits(cout, cin, tokens, split_k, sm, &w.kb_per_split);
+    count_tiles(d);
+    count_tiles(w);
+    int64_t grid;
+    return (plan_pair(pair, 2 * (int64_t)sm, &grid) ? 1 : 2) + (w.splits > 1 ? 1 : 0);
 }
 
 int jf_igemm_int32(const int8_t* a, const int8_t* b, int64_t M, int64_t N, int64_t K, int32_t* c, void* stream) {

@@ -81,9 +81,79 @@ __device__ __forceinline__ bool lean_wait(uint64_t* bar, uint32_t parity, volati
     return true;
 }
 
-template <bool A_MN, bool B_MN, int CONV>
+struct Item {        // tile and K range of a work item
+    uint32_t tile, split;
+    int kb0, kb1;
+    __device__ __forceinline__ Item(const GemmParams& p, uint32_t item) {
+        const uint32_t num_tiles = (uint32_t)(p.tiles_m * p.tiles_n);
+        tile = item % num_tiles;
+        split = item / num_tiles;
+        kb0 = (int)split * (int)p.kb_per_split;
+        kb1 = min((int)p.nkb, kb0 + (int)p.kb_per_split);
+    }
+};
+// The work items (tile, K range) of one CTA, in order.  SingleWalk: one GEMM, every gridDim.x-th item.
+template <bool A_MN>
+struct SingleWalk {
+    using Params = GemmParams;
+    const Params& p;
+    uint32_t item;
+    const uint32_t num_items;
+    __device__ __forceinline__ SingleWalk(const Params& p_, uint32_t cta)
+        : p(p_), item(cta), num_items((uint32_t)(p_.tiles_m * p_.tiles_n) * (uint32_t)p_.splits) {}
+    __device__ __forceinline__ bool valid() const { return item < num_items; }
+    __device__ __forceinline__ void next() { item += gridDim.x; }
+    __device__ __forceinline__ const GemmParams& gemm() const { return p; }
+    static __device__ __forceinline__ bool second() { return false; }
+    static __device__ __forceinline__ bool a_mn() { return A_MN; }
+    __device__ __forceinline__ void store(const uint64_t (&acc)[16], int64_t row, int64_t col, int64_t rowblk, int64_t colblk, int64_t split, int lane) const {
+        store_block<STORE_DENSE | STORE_QUANTISED>(p, acc, row, col, rowblk, colblk, split, lane);
+    }
+};
+// PairWalk: both gradients of a linear layer in one launch, the one with the longer K loop per item ("long") before the other.  Run one
+// after the other, each ends with CTA slots idle in its last round (dY 12288 x 2304, W 2304 x 768: 216 weight-gradient tiles of 384 K
+// blocks on 296 slots).  Here a CTA takes its long items round-robin; the CTAs that get one less than the others take `level` short items
+// in its place; the rest of the short items goes round-robin, first to those CTAs.  Fixed lists, no counter: a tile costs the same
+// wherever it runs.  Both gradients in us, two launches -> one: 12288 x 2304 x 768 169 -> 151, 7392 x 1600 x 1600 152 -> 136.
+// The epilogue names dX's and dW's parameters statically: with a run-time index the Philox round keys are loads, no longer operands.
+struct PairWalk {
+    using Params = GemmPair;
+    const Params& p;
+    const uint32_t cta;
+    uint32_t seq = 0, item = 0, which = 0;      // which: 0 dX, 1 dW
+    bool ok = false;
+    __device__ __forceinline__ PairWalk(const Params& p_, uint32_t cta_) : p(p_), cta(cta_) { locate(); }
+    __device__ __forceinline__ void locate() {
+        const uint32_t ctas = gridDim.x, short_from = p.short_from;             // CTAs from short_from on have one long item less
+        const uint32_t longs = p.rounds + (cta < short_from ? 1u : 0u);
+        if (seq < longs) {
+            which = p.long_one;
+            item = cta + seq * ctas;
+            ok = true;
+            return;
+        }
+        which = p.long_one ^ 1u;
+        const uint32_t q = seq - longs, level = cta >= short_from ? p.level : 0u;
+        if (q < level) item = cta - short_from + (ctas - short_from) * q;
+        else item = (ctas - short_from) * p.level + (cta >= short_from ? cta - short_from : cta + ctas - short_from) + ctas * (q - level);
+        ok = item < p.short_items;
+    }
+    __device__ __forceinline__ bool valid() const { return ok; }
+    __device__ __forceinline__ void next() { ++seq; locate(); }
+    __device__ __forceinline__ const GemmParams& gemm() const { return p.g[which]; }
+    __device__ __forceinline__ bool second() const { return which != 0u; }
+    __device__ __forceinline__ bool a_mn() const { return which != 0u; }
+    __device__ __forceinline__ void store(const uint64_t (&acc)[16], int64_t row, int64_t col, int64_t rowblk, int64_t colblk, int64_t split, int lane) const {
+        if (which == 0u) store_block<STORE_QUANTISED>(p.g[0], acc, row, col, rowblk, colblk, split, lane);
+        else store_block<STORE_DENSE>(p.g[1], acc, row, col, rowblk, colblk, split, lane);
+    }
+};
+
+// map_b1: dW's B operand (PairWalk; both gradients have the same A operand)
+template <class Walk, bool B_MN, int CONV>
 __global__ void __launch_bounds__(GEMM_THREADS, 2)
-gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
+gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_b1,
+            const __grid_constant__ typename Walk::Params params) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     // barriers: pair_full[2] at 0, pair_empty[2] at 16, abort flag at 32, tmem slot at 36, drain at 40, full[STAGES] at 48,
@@ -114,27 +184,27 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t block_x = blockIdx.x + grid_dependency();      // barriers and tensor memory are set up while the previous kernel ends
-    const uint32_t num_tiles = (uint32_t)(p.tiles_m * p.tiles_n), num_items = num_tiles * (uint32_t)p.splits;
-    const int nkb = (int)p.nkb, per = (int)p.kb_per_split;
 
     if (warp == CONSUMER_WARPS) {
         // ------------------------------------------------------------------ producer
         if (ptx::elect_one()) {
             uint32_t it = 0, s = 0, ph = 0;
             bool ok = true;
-            for (uint32_t item = block_x; item < num_items && ok; item += gridDim.x) {
-                const uint32_t tile = item % num_tiles, split = item / num_tiles;
+            for (Walk w(params, block_x); w.valid() && ok; w.next()) {
+                const GemmParams& p = w.gemm();
+                const Item i(p, w.item);
                 int tm, tn;
-                tile_coords(tile, (uint32_t)p.tiles_m, (uint32_t)p.tiles_n, tm, tn);
-                const int kb0 = (int)split * per, kb1 = min(nkb, kb0 + per);
+                tile_coords(i.tile, (uint32_t)p.tiles_m, (uint32_t)p.tiles_n, tm, tn);
+                const bool a_mn = w.a_mn();
+                const CUtensorMap* mb = w.second() ? &map_b1 : &map_b;
                 const int row = tm * BM, col = tn * BN;
-                for (int kb = kb0; kb < kb1; kb += KB_PER_STAGE) {
+                for (int kb = i.kb0; kb < i.kb1; kb += KB_PER_STAGE) {
                     if (!(ok = lean_wait(&empty_bar[s], ph ^ 1u, abort_flag, 1))) break;
                     ptx::mbar_arrive_expect_tx(&full_bar[s], STAGE_BYTES);
                     uint8_t* a = smem + s * STAGE_BYTES;
                     const int k = kb * QB;
-                    ptx::tma_load_2d(a, &map_a, &full_bar[s], A_MN ? row : k, A_MN ? k : row);
-                    ptx::tma_load_2d(a + A_BYTES, &map_b, &full_bar[s], B_MN ? col : k, B_MN ? k : col);
+                    ptx::tma_load_2d(a, &map_a, &full_bar[s], a_mn ? row : k, a_mn ? k : row);
+                    ptx::tma_load_2d(a + A_BYTES, mb, &full_bar[s], B_MN ? col : k, B_MN ? k : col);
                     ++it;
                     if (++s == STAGES) { s = 0; ph ^= 1u; }
                 }
@@ -144,20 +214,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         }
     } else if (warp == CONSUMER_WARPS + 1) {
         // ------------------------------------------------------------------ MMA issuer
-        constexpr uint32_t idesc = ptx::make_idesc_i8(BM, BN, A_MN, B_MN);
         uint32_t s = 0, ph = 0, par = 1;
         bool ok = true;
-        const uint64_t da_base = ptx::make_smem_desc_sw128(ptx::smem_u32(smem), A_MN ? 128 * 128 : 16, 1024);
         const uint64_t db_base = B_MN ? ptx::make_smem_desc_sw64(ptx::smem_u32(smem + A_BYTES), 128 * 64, 512)
                                       : ptx::make_smem_desc_sw128(ptx::smem_u32(smem + A_BYTES), 16, 1024);
-        for (uint32_t item = block_x; item < num_items && ok; item += gridDim.x) {
-            const uint32_t split = item / num_tiles;
-            const int kb0 = (int)split * per, kb1 = min(nkb, kb0 + per);
-            for (int kb = kb0; kb < kb1 && ok; kb += KB_PER_STAGE) {
+        for (Walk w(params, block_x); w.valid() && ok; w.next()) {
+            const Item i(w.gemm(), w.item);
+            const bool a_mn = w.a_mn();
+            const uint32_t idesc = a_mn ? ptx::make_idesc_i8(BM, BN, true, B_MN) : ptx::make_idesc_i8(BM, BN, false, B_MN);
+            const uint64_t da_base = ptx::make_smem_desc_sw128(ptx::smem_u32(smem), a_mn ? 128 * 128 : 16, 1024);
+            const uint32_t a_step = a_mn ? 256 : 2;         // descriptor units (16 bytes) from one K block to the next
+            for (int kb = i.kb0; kb < i.kb1 && ok; kb += KB_PER_STAGE) {
                 if (!(ok = __all_sync(0xffffffffu, lean_wait(&full_bar[s], ph, abort_flag, 2)))) break;
                 ptx::tc_fence_after();
                 const uint64_t da = da_base + (uint64_t)(s * (STAGE_BYTES / 16)), db = db_base + (uint64_t)(s * (STAGE_BYTES / 16));
-                const int nblk = min(KB_PER_STAGE, kb1 - kb);
+                const int nblk = min(KB_PER_STAGE, i.kb1 - kb);
 #pragma unroll
                 for (int pp = 0; pp < 2; ++pp) {
                     if (!(ok = __all_sync(0xffffffffu, lean_wait(&pair_empty[pp], par, abort_flag, 3)))) break;
@@ -166,7 +237,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 #pragma unroll
                         for (int j = 2 * pp; j < 2 * pp + 2; ++j)
                             if (j < nblk)
-                                ptx::umma_i8(tmem_base + j * BN, da + (uint64_t)(A_MN ? j * 256 : j * 2),
+                                ptx::umma_i8(tmem_base + j * BN, da + (uint64_t)(j * a_step),
                                              db + (uint64_t)(B_MN ? j * 128 : j * 2), idesc, 0u);
                         ptx::umma_commit(&pair_full[pp]);       // a pair without a K block is passed on empty: every tile starts at pair 0
                         if (pp == 1) ptx::umma_commit(&empty_bar[s]);
@@ -187,11 +258,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         const uint32_t base = ptx::smem_u32(bars);
         const uint32_t t0 = tmem_base + ((uint32_t)(quad * 32) << 16) + cg * 32;
         uint32_t par = 0;
-        for (uint32_t item = block_x; item < num_items; item += gridDim.x) {
-            const uint32_t tile = item % num_tiles, split = item / num_tiles;
+        for (Walk w(params, block_x); w.valid(); w.next()) {
+            const GemmParams& p = w.gemm();
+            const Item item(p, w.item);
             int tm, tn;
-            tile_coords(tile, (uint32_t)p.tiles_m, (uint32_t)p.tiles_n, tm, tn);
-            const int kb0 = (int)split * per, n = min(nkb, kb0 + per) - kb0;
+            tile_coords(item.tile, (uint32_t)p.tiles_m, (uint32_t)p.tiles_n, tm, tn);
+            const int kb0 = item.kb0, n = item.kb1 - kb0;
             const int rowblk = tm * (BM / QB) + quad, colblk = tn * (BN / QB) + cg;
             const bool blk_ok = rowblk < (int)(p.M / QB) && colblk < (int)(p.N / QB);   // warp-uniform
 
@@ -276,7 +348,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 par ^= 1u;
             }
             if (!blk_ok) continue;
-            store_block(p, acc, (int64_t)rowblk * QB + lane, (int64_t)colblk * QB, rowblk, colblk, split, lane);
+            w.store(acc, (int64_t)rowblk * QB + lane, (int64_t)colblk * QB, rowblk, colblk, item.split, lane);
         }
     }
     ptx::tc_fence_before();

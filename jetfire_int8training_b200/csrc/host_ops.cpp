@@ -380,22 +380,28 @@ PyObject* linear_forward(PyObject* const* a) {
     return quantised ? tuple(std::move(y), std::move(sy)) : wrap(std::move(y));
 }
 
-Tensor wgrad(const Mat& x, const Scale& sx, const Mat& g, const Scale& sg, at::ScalarType dt, int split_k) {
-    const int64_t T = g.M, cout = g.N, cin = x.N;
-    const int splits = jf_igemm_wgrad_plan(cout, cin, T, split_k);
-    if (splits < 1) check(splits, "int8_linear_wgrad(plan)");
-    Tensor dw = empty({cout, cin}, dt, g.t), scratch;
-    if (splits > 1) scratch = empty({splits * cout * cin}, at::kFloat, g.t);
-    check(jf_igemm_wgrad(i8(g), 0, i8(x), sg.t.const_data_ptr(), sg.cols, 1, sx.t.const_data_ptr(), sx.cols, 1, cout, cin, T,
-                         dt == at::kHalf ? JF_F16 : JF_F32, dw.mutable_data_ptr(), splits, splits > 1 ? scratch.mutable_data_ptr<float>() : nullptr,
-                         nullptr, 0, stream()), "int8_linear_wgrad");
-    return dw;
-}
+// dW and the workspace of its split sum
+struct Wgrad {
+    Tensor dw, scratch;
+    int dtype, splits;
+    Wgrad(const Mat& x, const Mat& g, bool fp16, int split_k) : dtype(fp16 ? JF_F16 : JF_F32) {
+        const int64_t cout = g.N, cin = x.N;
+        splits = jf_igemm_wgrad_plan(cout, cin, g.M, split_k);
+        if (splits < 1) check(splits, "int8_linear_wgrad(plan)");
+        dw = empty({cout, cin}, fp16 ? at::kHalf : at::kFloat, g.t);
+        if (splits > 1) scratch = empty({splits * cout * cin}, at::kFloat, g.t);
+    }
+    float* workspace() const { return splits > 1 ? scratch.mutable_data_ptr<float>() : nullptr; }
+};
 
 // linear_wgrad(x, sx, g, sg, fp16, split_k)
 PyObject* linear_wgrad(PyObject* const* a) {
     const Mat x = payload(a[0]), g = payload(a[2]);
-    return wrap(wgrad(x, scale_arg(a[1]), g, scale_arg(a[3]), bool_arg(a[4]) ? at::kHalf : at::kFloat, (int)int_arg(a[5])));
+    const Scale sx = scale_arg(a[1]), sg = scale_arg(a[3]);
+    Wgrad w(x, g, bool_arg(a[4]), (int)int_arg(a[5]));
+    check(jf_igemm_wgrad(i8(g), 0, i8(x), sg.t.const_data_ptr(), sg.cols, 1, sx.t.const_data_ptr(), sx.cols, 1, g.N, x.N, g.M, w.dtype,
+                         w.dw.mutable_data_ptr(), w.splits, w.workspace(), nullptr, 0, stream()), "int8_linear_wgrad");
+    return wrap(std::move(w.dw));
 }
 
 // linear_backward(x, sx, g, sg, w, sw, quantised, wgrad_fp16, split_k, stochastic, noise, seed, offset)
@@ -404,7 +410,7 @@ PyObject* linear_backward(PyObject* const* a) {
     const Tensor& sg_in = cuda_arg(a[3]);
     const Scale sx = scale_arg(a[1]), sg = scale_arg(a[3]), sw = scale_arg(a[5]);
     const int64_t cout = w.t.size(0), cin = w.N, M = g.M;
-    const char* what = "int8_linear_backward(dgrad)";
+    const char* what = "int8_linear_backward";
     if (M <= 0 || M % 32 || cin <= 0 || cin % 32 || cout <= 0 || cout % 32) check(JF_ERR_SHAPE, what);
     if (g.N != cout || x.N != cin) fail(PyExc_RuntimeError, "int8_linear_backward: the last dimensions do not fit the weight");
     const bool quantised = bool_arg(a[6]);
@@ -414,11 +420,12 @@ PyObject* linear_backward(PyObject* const* a) {
     Tensor gx = out_last(tensor_arg(a[2]), cin, quantised ? at::kChar : at::kHalf);
     Tensor gsx = quantised ? out_last(sg_in, cin / 32, at::kHalf) : Tensor();
     if (quantised && gsx.numel() != (M / 32) * (cin / 32)) fail(PyExc_RuntimeError, "the scales do not fit the payload");
-    check(jf_igemm_dgrad(i8(g), i8(w), sg.t.const_data_ptr(), sg.cols, 1, sw.t.const_data_ptr(), sw.cols, 1, M, cin, cout,
-                         quantised ? JF_OUT_INT8 : JF_OUT_DEQUANT_F16, quantised ? i8(gx) : nullptr, quantised ? gsx.mutable_data_ptr() : nullptr,
-                         quantised ? nullptr : gx.mutable_data_ptr(), sr.on, sr.ptr(), sr.seed, sr.offset, nullptr, 0, stream()), what);
-    Tensor gw = wgrad(x, sx, g, sg, bool_arg(a[7]) ? at::kHalf : at::kFloat, (int)int_arg(a[8]));
-    return quantised ? tuple(std::move(gx), std::move(gsx), std::move(gw)) : tuple(std::move(gx), std::move(gw));
+    Wgrad dw(x, g, bool_arg(a[7]), (int)int_arg(a[8]));
+    check(jf_igemm_backward(i8(g), i8(w), i8(x), sg.t.const_data_ptr(), sg.cols, 1, sw.t.const_data_ptr(), sw.cols, 1, sx.t.const_data_ptr(),
+                            sx.cols, 1, M, cout, cin, quantised ? JF_OUT_INT8 : JF_OUT_DEQUANT_F16, quantised ? i8(gx) : nullptr,
+                            quantised ? gsx.mutable_data_ptr() : nullptr, quantised ? nullptr : gx.mutable_data_ptr(), sr.on, sr.ptr(),
+                            sr.seed, sr.offset, dw.dtype, dw.dw.mutable_data_ptr(), dw.splits, dw.workspace(), stream()), what);
+    return quantised ? tuple(std::move(gx), std::move(gsx), std::move(dw.dw)) : tuple(std::move(gx), std::move(dw.dw));
 }
 
 // ------------------------------------------------------------------------------------------------ the GPT-2 caller's floating-point parts

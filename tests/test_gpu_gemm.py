@@ -150,6 +150,27 @@ def test_wgrad_split_k_is_deterministic_and_matches_oracle(LIN, L, oracle, op16,
         assert torch.equal(dw, LIN.int8_linear_wgrad(t(X), t(SX), t(G), t(SG), dt, split))
 
 
+# fewer items than CTAs; no full round of dW tiles; full rounds only (no levelling); dX items longer than dW's; split K; ragged tiles
+@pytest.mark.parametrize("tokens,cin,cout,split", [(32, 32, 32, 1), (96, 160, 2336, 0), (2048, 1184, 2048, 1), (128, 2368, 1024, 1),
+                                                   (4096, 96, 160, 3), (4128, 1600, 1600, 0)])
+@pytest.mark.parametrize("quantised,dt", [(True, torch.float32), (False, torch.float16)])
+def test_both_gradients_in_one_launch_equal_one_by_one(LIN, L, tokens, cin, cout, split, quantised, dt):
+    gen = torch.Generator(device=DEV).manual_seed(tokens + cin)
+    def operand(r, c):
+        return (torch.randint(-127, 128, (r, c), generator=gen, device=DEV, dtype=torch.int8),
+                (torch.rand(r // 32, c // 32, generator=gen, device=DEV) * 0.099 + 1e-3).half())
+    (G, SG), (W, SW), (X, SX) = operand(tokens, cout), operand(cout, cin), operand(tokens, cin)
+    *dx, dw = LIN.int8_linear_backward(X, SX, G, SG, None, W, SW, 32, True, quantised, sr_key=(3, 8), wgrad_split_k=split, wgrad_out_dtype=dt)
+    out = torch.empty((tokens, cin), dtype=torch.int8 if quantised else torch.float16, device=DEV)
+    so = torch.empty((tokens // 32, cin // 32), dtype=torch.float16, device=DEV)
+    rc = L.jf_igemm_dgrad(G.data_ptr(), W.data_ptr(), SG.data_ptr(), SG.stride(0), 1, SW.data_ptr(), SW.stride(0), 1, tokens, cin, cout,
+                          0 if quantised else 1, out.data_ptr(), so.data_ptr(), out.data_ptr(), 1, None, 3, 8, None, 0,
+                          torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    assert torch.equal(dx[0], out) and (not quantised or torch.equal(dx[1], so))
+    assert torch.equal(dw, LIN.int8_linear_wgrad(X, SX, G, SG, dt, split))
+
+
 def test_config1_linear_layer(LIN, oracle):
     """Single linear layer forward + backward on the benchmark's first configuration: X bf16 [2048,768] N(0,1) with 0.5% outlier
     channels x30, W bf16 [3072,768] N(0,0.02), dY N(0,1e-2) [2048,3072], all block-quantised, seed 0."""
