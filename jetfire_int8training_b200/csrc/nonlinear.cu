@@ -838,27 +838,30 @@ ln_fwd_kernel(const int8_t* __restrict__ qx, const __half* __restrict__ sx, cons
 // LayerNorm backward (dx and per-32-row partial dgamma), row reductions over the tile's 128-column slab.
 // Rounding points of the reference: mean, rstd, x, dy, xhat in fp16; c1, c2 and the dx expression in fp32; dx -> fp16.
 // =========================================================================================================
-// Two warps share one 32x128 slab tile, 64 columns each (64 values per lane instead of 128: 2 CTAs per SM instead of one
-// at 242 registers).  The quantisation blocks and the dgamma columns are private to a warp; only the two row sums per row cross
-// the warps, through shared memory and a 64-thread named barrier per row pass.  The sum order is the one of a single warp over
-// 8 lanes: ((l0+l1)+(l2+l3)) + ((l4+l5)+(l6+l7)).
-template <bool SR, int TW = 64>
-__global__ void __launch_bounds__(THREADS, 2)
+// A CTA is one 32x128 slab tile: two warps of 64 columns each (64 values per lane; 8 CTAs per SM at 128 registers).  The quantisation blocks
+// and the dgamma columns are private to a warp; the row sums cross the warps once per tile, through shared memory.  The sum order is the one
+// of a single warp over 8 lanes: ((l0+l1)+(l2+l3)) + ((l4+l5)+(l6+l7)).
+// What bounds it: issue (36 instructions per element) and the latency of the exchange at 16 warps per SM.  One exchange per row pass -- four
+// barriers per tile, 16 + 48 shuffles for the sums, eight divisions per lane -- and CTAs of four tiles, which wait for their slowest, left an
+// SM idle 19 % of the time.  The first loop therefore does all passes and keeps xhat and dy as fp16 pairs, the sums are handed out so that a
+// lane reduces what it needs (6 + 14 shuffles) and divides twice, and the second loop widens again: with dgamma 8192 x 1600 28.1 -> 26.6 us,
+// 12288 x 3072 74 -> 67, 16384 x 6400 190 -> 171.  (96 registers and 10 CTAs: 32 us; the payloads kept instead of the fp16 pairs: 31.)
+constexpr int LNB_THREADS = 64;
+template <bool SR>
+__global__ void __launch_bounds__(LNB_THREADS, 8)
 ln_bwd_kernel(const int8_t* __restrict__ qx, const __half* __restrict__ sx, const int8_t* __restrict__ qg,
               const __half* __restrict__ sg, const float* __restrict__ gamma, const float* __restrict__ mean,
               const float* __restrict__ rstd, int64_t M, int64_t N, int8_t* __restrict__ qd, __half* __restrict__ sd,
               float* __restrict__ dw_partial, SrCfg sr) {
-    const uint32_t block_x = blockIdx.x + grid_dependency();
-    constexpr int NP = Geo<TW>::NP, WPS = 128 / TW, PAIRS = WARPS / WPS;   // WPS warps per slab tile, PAIRS slab tiles per CTA
-    __shared__ float2 row_part[PAIRS][WPS][QB];        // [slab tile][part][row of the tile] = (sum xhat*wdy, sum wdy) over the part
-    const int warp = threadIdx.x >> 5, pair = warp / WPS, half = warp % WPS;
-    const int64_t slabs_n = (N + 127) / 128, tiles_n_ = (N + TW - 1) / TW;
-    const int64_t slab_tile = (int64_t)block_x * PAIRS + pair;          // index of the 32 x 128 slab tile
-    if (slab_tile >= (M / QB) * slabs_n) return;                           // both warps of a pair leave together
-    const int64_t tm_ = (int64_t)((uint32_t)slab_tile / (uint32_t)slabs_n);                      // 32-bit division
-    const int64_t tn_ = (int64_t)((uint32_t)slab_tile % (uint32_t)slabs_n) * WPS + half;
+    const uint32_t slab_tile = blockIdx.x + grid_dependency();             // index of the 32 x 128 slab tile
+    constexpr int TW = 64, NP = Geo<TW>::NP;
+    static_assert(NP == 4 && Geo<TW>::LPR == 4, "a lane of a row's four ends up with the sums of one of the four passes");
+    __shared__ float2 row_part[2][QB];                 // [half][row of the tile] = (sum xhat*wdy, sum wdy) over the half's 64 columns
+    const int half = threadIdx.x >> 5;
+    const uint32_t slabs_n = (uint32_t)((N + 127) / 128);
+    const int64_t tiles_n_ = (N + TW - 1) / TW, tn_ = (int64_t)(slab_tile % slabs_n) * 2 + half;
     // the right half of a short last slab may lie outside the tensor: such a warp loads zeros and only takes part in the sums
-    Tile t = make_tile<TW>(tm_ * tiles_n_ + (tn_ < tiles_n_ ? tn_ : tiles_n_ - 1), tiles_n_, N);
+    Tile t = make_tile<TW>((int64_t)(slab_tile / slabs_n) * tiles_n_ + (tn_ < tiles_n_ ? tn_ : tiles_n_ - 1), tiles_n_, N);
     if (tn_ >= tiles_n_) t.active = false;
     int4 rx[NP], rgr[NP];
     load_rows<TW>(qx, t, N, rx);
@@ -871,89 +874,101 @@ ln_bwd_kernel(const int8_t* __restrict__ qx, const __half* __restrict__ sx, cons
 #pragma unroll
         for (int j = 0; j < 16; ++j) gm[j] = 0.f;
     }
-    const float n_f = (float)N;
     uint64_t gm2[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) gm2[j] = f2_pack(gm[2 * j], gm[2 * j + 1]);
-    __half2 v16[NP][8];    // dx, rounded to fp16 (kept packed: half the registers, and the block absmax takes two values per instruction)
+    __half2 xhat[NP][8], dy[NP][8];
     uint64_t dwp2[8];      // partial dgamma over this lane's rows
 #pragma unroll
     for (int j = 0; j < 8; ++j) dwp2[j] = 0ull;
+    float s1[NP], s2[NP], rs[NP];
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
         const int64_t row = row_of<TW>(t, i);
-        const int row_in_tile = i * Geo<TW>::RPP + t.rg;
         const __half2 mu2 = __half2half2(__float2half_rn(__ldg(mean + row)));
         const __half rs16 = __float2half_rn(__ldg(rstd + row));
         const __half2 rs2 = __half2half2(rs16);
-        const float rs = __half2float(rs16);
-        uint64_t xh2[8], wdy2[8];
+        rs[i] = __half2float(rs16);
         __half2 hx[8], hg[8];
         unpack16_h2(rx[i], hx);
         unpack16_h2(rgr[i], hg);
-        float s1 = 0.f, s2 = 0.f;
+        s1[i] = 0.f;
+        s2[i] = 0.f;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const __half2 x16 = __hmul2_rn(hx[j], sx2);
-            const __half2 dy16 = __hmul2_rn(hg[j], sg2);
-            const __half2 xhat16 = __hmul2_rn(__hsub2_rn(x16, mu2), rs2);
-            const float2 xf = __half22float2(xhat16), dyf = __half22float2(dy16), pr = __half22float2(__hmul2_rn(dy16, xhat16));
-            xh2[j] = f2_pack(xf.x, xf.y);
-            wdy2[j] = f2_mul(gm2[j], f2_pack(dyf.x, dyf.y));
+            dy[i][j] = __hmul2_rn(hg[j], sg2);
+            xhat[i][j] = __hmul2_rn(__hsub2_rn(__hmul2_rn(hx[j], sx2), mu2), rs2);
+            const float2 xf = __half22float2(xhat[i][j]), dyf = __half22float2(dy[i][j]), pr = __half22float2(__hmul2_rn(dy[i][j], xhat[i][j]));
+            const uint64_t wdy2 = f2_mul(gm2[j], f2_pack(dyf.x, dyf.y));
             float p0, p1, w0, w1;
-            f2_unpack(f2_mul(xh2[j], wdy2[j]), p0, p1);
-            f2_unpack(wdy2[j], w0, w1);
-            s1 = __fadd_rn(__fadd_rn(s1, p0), p1);
-            s2 = __fadd_rn(__fadd_rn(s2, w0), w1);
+            f2_unpack(f2_mul(f2_pack(xf.x, xf.y), wdy2), p0, p1);
+            f2_unpack(wdy2, w0, w1);
+            s1[i] = __fadd_rn(__fadd_rn(s1[i], p0), p1);
+            s2[i] = __fadd_rn(__fadd_rn(s2[i], w0), w1);
             dwp2[j] = f2_add(dwp2[j], f2_pack(pr.x, pr.y));
         }
-        // sums over this warp's 64 columns, then the other warp's through shared memory (left + right)
-        s1 = row_sum<TW>(s1);
-        s2 = row_sum<TW>(s2);
-        if (t.cc == 0) row_part[pair][half][row_in_tile] = make_float2(s1, s2);
-        asm volatile("bar.sync %0, %1;" ::"r"(1 + pair), "n"(32 * WPS) : "memory");
-        float2 tot;
-        {
-            const float2 lft = row_part[pair][0][row_in_tile], rgt = row_part[pair][1][row_in_tile];
-            tot = make_float2(__fadd_rn(lft.x, rgt.x), __fadd_rn(lft.y, rgt.y));
-            if (WPS == 4) {
-                const float2 l2 = row_part[pair][2][row_in_tile], r2 = row_part[pair][3][row_in_tile];
-                tot = make_float2(__fadd_rn(tot.x, __fadd_rn(l2.x, r2.x)), __fadd_rn(tot.y, __fadd_rn(l2.y, r2.y)));
-            }
-        }
-        const float c1 = __fdiv_rn(tot.x, n_f), c2 = __fdiv_rn(tot.y, n_f);
-        const uint64_t nc1 = f2_pack(-c1, -c1), nc2 = f2_pack(-c2, -c2), rs_2 = f2_pack(rs, rs);
-#pragma unroll
-        for (int j = 0; j < 16; j += 2) {
-            // (wdy - (xhat * c1 + c2)) * rstd, each operation rounded:  -(a*b + c) == (a * -b) + -c  exactly
-            const uint64_t ntt = f2_add(f2_mul(xh2[j / 2], nc1), nc2);
-            float d0, d1;
-            f2_unpack(f2_mul(f2_add(wdy2[j / 2], ntt), rs_2), d0, d1);
-            v16[i][j / 2] = __floats2half2_rn(d0, d1);
-        }
     }
-    // partial dgamma: reduce the row groups, lanes with rg == 0 write 16 columns
-    float dwp[16];
+    // Row sums over this warp's 64 columns, (l0 + l1) + (l2 + l3) over a row's lanes: each step hands half of the passes to the partner, and
+    // lane cc ends up with pass cc.  Then left half + right half through shared memory, and the two quotients.
+    const bool b0 = t.cc & 1, b1 = t.cc & 2;
+    auto over_row = [&](const float (&v)[NP]) {
+        const float e0 = __fadd_rn(b0 ? v[1] : v[0], __shfl_xor_sync(0xffffffffu, b0 ? v[0] : v[1], 1));
+        const float e1 = __fadd_rn(b0 ? v[3] : v[2], __shfl_xor_sync(0xffffffffu, b0 ? v[2] : v[3], 1));
+        return __fadd_rn(b1 ? e1 : e0, __shfl_xor_sync(0xffffffffu, b1 ? e0 : e1, 2));
+    };
+    const float r1 = over_row(s1), r2 = over_row(s2);
+    const int my_row = t.cc * Geo<TW>::RPP + t.rg;
+    row_part[half][my_row] = make_float2(r1, r2);
+    __syncthreads();
+    // partial dgamma: (..(r0 + r1) + (r2 + r3)..) over the row groups in the same way; a lane ends up with two of its 16 columns
+    {
+        float a[16], b[8], c[4], e[2];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) f2_unpack(dwp2[j], dwp[2 * j], dwp[2 * j + 1]);
+        for (int j = 0; j < 8; ++j) f2_unpack(dwp2[j], a[2 * j], a[2 * j + 1]);
+        const bool g0 = t.rg & 1, g1 = t.rg & 2, g2 = t.rg & 4;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) dwp[j] = col_sum<TW>(dwp[j]);
-    if (t.active && t.rg == 0) {
-        float4* dst = reinterpret_cast<float4*>(dw_partial + t.tm * N + t.col);
+        for (int j = 0; j < 8; ++j) b[j] = __fadd_rn(g0 ? a[8 + j] : a[j], __shfl_xor_sync(0xffffffffu, g0 ? a[j] : a[8 + j], 4));
 #pragma unroll
-        for (int k = 0; k < 4; ++k) dst[k] = make_float4(dwp[4 * k], dwp[4 * k + 1], dwp[4 * k + 2], dwp[4 * k + 3]);
+        for (int j = 0; j < 4; ++j) c[j] = __fadd_rn(g1 ? b[4 + j] : b[j], __shfl_xor_sync(0xffffffffu, g1 ? b[j] : b[4 + j], 8));
+#pragma unroll
+        for (int j = 0; j < 2; ++j) e[j] = __fadd_rn(g2 ? c[2 + j] : c[j], __shfl_xor_sync(0xffffffffu, g2 ? c[j] : c[2 + j], 16));
+        if (t.active) *reinterpret_cast<float2*>(dw_partial + t.tm * N + t.col + (g0 ? 8 : 0) + (g1 ? 4 : 0) + (g2 ? 2 : 0)) = make_float2(e[0], e[1]);
     }
-    __half2 m2 = __floats2half2_rn(0.f, 0.f);
+    const float2 lft = row_part[0][my_row], rgt = row_part[1][my_row];
+    const float n_f = (float)N;
+    const float c1 = __fdiv_rn(__fadd_rn(lft.x, rgt.x), n_f), c2 = __fdiv_rn(__fadd_rn(lft.y, rgt.y), n_f);
+    // (opaque to the compiler, which would otherwise keep the widened values of the first loop in twice the registers)
 #pragma unroll
     for (int i = 0; i < NP; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) m2 = __hmax2(m2, __habs2(v16[i][j]));
+        for (int j = 0; j < 8; ++j) {
+            asm volatile("" : "+r"(*reinterpret_cast<uint32_t*>(&xhat[i][j])));
+            asm volatile("" : "+r"(*reinterpret_cast<uint32_t*>(&dy[i][j])));
+        }
+    __half2 m2 = __floats2half2_rn(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+        const float n1 = -__shfl_sync(0xffffffffu, c1, i, 4), n2 = -__shfl_sync(0xffffffffu, c2, i, 4);
+        const uint64_t nc1 = f2_pack(n1, n1), nc2 = f2_pack(n2, n2), rs_2 = f2_pack(rs[i], rs[i]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            // (wdy - (xhat * c1 + c2)) * rstd with the inner sum rounded once (-(a*b + c) == fma(a, -b, -c)) and every other operation by itself.
+            // wdy is a scalar product: the assembler contracts a packed product with the packed sum that is its only use.
+            const float2 xf = __half22float2(xhat[i][j]), dyf = __half22float2(dy[i][j]);
+            float g0, g1, d0, d1;
+            f2_unpack(gm2[j], g0, g1);
+            const uint64_t ntt = f2_fma(f2_pack(xf.x, xf.y), nc1, nc2);
+            f2_unpack(f2_mul(f2_add(f2_pack(__fmul_rn(g0, dyf.x), __fmul_rn(g1, dyf.y)), ntt), rs_2), d0, d1);
+            xhat[i][j] = __floats2half2_rn(d0, d1);            // dx, rounded to fp16, in xhat's place
+            m2 = __hmax2(m2, __habs2(xhat[i][j]));
+        }
+    }
     const float2 mf = __half22float2(m2);
     const float scale32 = __fdiv_rn(block_max<TW>(fmaxf(mf.x, mf.y)), 127.0f);
     emit_quantized<TW, SR, false>([&](int i, float (&a)[16]) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const float2 f = __half22float2(v16[i][j]);
+            const float2 f = __half22float2(xhat[i][j]);
             a[2 * j] = f.x; a[2 * j + 1] = f.y;
         }
     }, scale32, t, M, N, qd, sd, sr, nullptr, nullptr);
@@ -1545,10 +1560,11 @@ int jf_int8_layernorm_backward(const int8_t* qx, const void* sx, const int8_t* q
     cudaStream_t st = (cudaStream_t)stream;
     SrCfg sr = make_sr(noise, seed, offset, M, N);
     const int64_t slab_tiles = (M / QB) * ((N + 127) / 128);
-    const unsigned grid = (unsigned)((slab_tiles + WARPS / 2 - 1) / (WARPS / 2));   // two warps per 32 x 128 slab tile
+    if (slab_tiles >= (int64_t(1) << 31)) return JF_ERR_SHAPE;
+    const unsigned grid = (unsigned)slab_tiles;
     const __half* sxh = (const __half*)sx; const __half* sgh = (const __half*)sg; __half* sdh = (__half*)sd;
-    if (stochastic) jf::launch(ln_bwd_kernel<true>, grid, THREADS, 0, st, qx, sxh, qg, sgh, gamma, mean, rstd, M, N, qd, sdh, scratch, sr);
-    else jf::launch(ln_bwd_kernel<false>, grid, THREADS, 0, st, qx, sxh, qg, sgh, gamma, mean, rstd, M, N, qd, sdh, scratch, sr);
+    if (stochastic) jf::launch(ln_bwd_kernel<true>, grid, LNB_THREADS, 0, st, qx, sxh, qg, sgh, gamma, mean, rstd, M, N, qd, sdh, scratch, sr);
+    else jf::launch(ln_bwd_kernel<false>, grid, LNB_THREADS, 0, st, qx, sxh, qg, sgh, gamma, mean, rstd, M, N, qd, sdh, scratch, sr);
     if (int e = check_launch()) return e;
     jf::launch(ln_bwd_dw_kernel, (unsigned)((N + 31) / 32), 256, 0, st, scratch, M / QB, N, dgamma);
     return check_launch();
